@@ -501,6 +501,7 @@ PlanObj::Workspace& acquire_workspace(PlanObj& P, uint64_t need, cudaStream_t s)
     if (grow->ptr) ck(cudaFree(grow->ptr), "cudaFree(workspace)");
     grow->ptr = nullptr;
     grow->bytes = 0;
+    grow->zeroed = false;
     ck(cudaMalloc(&grow->ptr, need), "cudaMalloc(workspace)");
     grow->bytes = need;
     return *grow;
@@ -537,8 +538,12 @@ AG_EXPORT int aether_plan_launch(void* plan, const AetherLaunch* a, void* stream
                 PlanObj::Workspace& w = acquire_workspace(*P, need, s);
                 k.ws = static_cast<char*>(w.ptr);
                 k.ws_bytes = w.bytes;
-                ck(cudaMemsetAsync(k.ws, 0, 16, s), "cudaMemsetAsync(counter)");
+                // every launch leaves the counter at 0, so only the first one on a
+                // new entry clears it (a caller's own workspace is cleared each time)
+                if (!w.zeroed) ck(cudaMemsetAsync(k.ws, 0, 16, s), "cudaMemsetAsync(counter)");
+                w.zeroed = false;
                 launch_plan_kernel(*P, k, a->n, vect, s);
+                w.zeroed = true;
                 // the entry is busy until this event completes, except for
                 // later launches on the same stream, which run after it
                 ck(cudaEventRecord(w.done, s), "cudaEventRecord(workspace)");

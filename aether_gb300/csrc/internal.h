@@ -59,6 +59,7 @@ struct PlanObj {
         cudaStream_t last_stream = nullptr;
         bool ordered = false;          // last_stream orders later launches on it
         cudaEvent_t done = nullptr;    // recorded after the last launch
+        bool zeroed = false;           // the counter is 0 once the entry's launches so far have ended
     };
     std::mutex ws_mu;
     std::vector<Workspace> ws;

@@ -1223,20 +1223,19 @@ std::string generate_source(const Plan& plan_in, const Lowering& low, const std:
         k << "extern \"C\" __global__ void " << lb << " " << name << "(const AgArgs a) {\n";
         k << "    const ag_u64 per = (ag_u64)AG_BLOCK * AG_IPT * " << V << ";\n";
         k << "    const ag_u64 nchunks = (a.n + per - 1) / per;\n";
+        if (sum) k << "    double h = 0.0, c = 0.0;\n";   // the thread's pair over all its chunks
         k << "    for (ag_u64 ch = blockIdx.x; ch < nchunks; ch += gridDim.x) {\n";
         if (sum && prec) {
-            // float-float per thread, FP64 from the warp tree on
+            // float-float within a chunk, an FP64 pair across chunks
             k << "        ag::e64::df acc = ag::e64::mk(0.0f, 0.0f);\n";
             k << "        ag_chunk<" << V << ">(a, ch, acc);\n";
-            k << "        ag::sum_chunk_finish<AG_BLOCK>(a, ch, nchunks, ag::e64::f2d(acc.hi), ag::e64::f2d(acc.lo));\n";
+            k << "        ag::pair_combine(h, c, ag::e64::f2d(acc.hi), ag::e64::f2d(acc.lo), h, c);\n";
         } else if (sum) {
-            k << "        double h = 0.0, c = 0.0;\n";
             k << "        ag_chunk<" << V << ">(a, ch, h, c);\n";
-            k << "        ag::sum_chunk_finish<AG_BLOCK>(a, ch, nchunks, h, c);\n";
         } else {
             k << "        ag_chunk<" << V << ">(a, ch);\n";
         }
-        k << "    }\n}\n";
+        k << (sum ? "    }\n    ag::sum_finish<AG_BLOCK>(a, h, c);\n}\n" : "    }\n}\n");
     }
     return k.str();
 }
