@@ -305,8 +305,9 @@ class Launch:
 def prepare(dst, expr, op="set", n=None, sample_offset=0, reduce_out=None, workspace=None, tune=False, **low):
     """Lower `dst <op>= expr` and bind its arguments; returns a Launch.
 
-    Lowering keywords (include/aether_gb300.h AetherLowering): math = 0 FP64
-    on the FP64 pipe, 1 double-float FP64 emulation (about 48 bits), 2 the
+    Lowering keywords (include/aether_gb300.h AetherLowering): math = 0 native
+    FP64 (FP64 arithmetic; division, roots, exp, logarithms, sine, cosine and
+    normal draws rounded from triple-float), 1 double-float FP64 emulation (about 48 bits), 2 the
     precision form (f32/ff storage, float-float arithmetic), 3 FP64-grade
     triple-float on the FP32/INT pipes (f64 plans, the FP64 contract);
     contract (FMA contraction), block, ipt, vec, min_blocks.

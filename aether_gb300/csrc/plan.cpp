@@ -394,6 +394,18 @@ std::string ctype_of(DType d) {
     }
 }
 
+// Native FP64 code (an f64 plan at math 0, or the native lanes of an emulated
+// plan) that divides, takes a root, exp, log, sine or cosine, or draws a normal
+// gets these from ag::n64 (AG_NATIVE_TF): the FP64 pipe's own are slower at
+// every size, 2 to 9 times (ag_tf64.cuh).
+bool native_needs_tf(const Plan& P) {
+    static const std::set<std::string> ops = {"sqrt", "rsqrt", "exp", "log", "log1p", "sin", "cos", "div", "unit", "norm",
+                                              "rnorm", "inv", "normal", "lognormal", "exponential"};
+    for (const Node& n : P.nodes)
+        if (ops.count(n.op)) return true;
+    return false;
+}
+
 struct Gen {
     const Plan& P;
     const Lowering& L;
@@ -448,6 +460,19 @@ struct Gen {
         if (tfm) kSafeLo = -80;
         W = tfm ? "ag::t64::tf" : dfm ? "ag::e64::df" : ((P.dst_dtype == DType::F64 || force_double) ? "double" : "float");
         S = P.dst_dtype == DType::F64 ? "double" : "float";
+        xfma = W == "double" && L.contract && native_needs_tf(P);
+    }
+
+    // Contraction in native code that calls ag::n64, written out: those
+    // functions branch, and the compiler contracts within a block only, so the
+    // same tree would round differently in a plan's kernel and in a batch. A
+    // sum takes its first product operand, else its second, into an FMA (the
+    // compiler's own order). `prods` maps a product's spelling to its factors.
+    bool xfma = false;
+    mutable std::map<std::string, std::pair<std::string, std::string>> prods;
+    const std::pair<std::string, std::string>* product(const std::string& v) const {
+        const auto it = prods.find(v);
+        return it == prods.end() ? nullptr : &it->second;
     }
 
     // A double-float value that is an exact float (an f32 operand): products
@@ -492,10 +517,20 @@ struct Gen {
 
     std::string add(const std::string& a, const std::string& b) const {
         if (dfm) return NS + "add(" + a + ", " + b + ")";
+        if (xfma) {
+            if (const auto* p = product(a)) return "__fma_rn(" + p->first + ", " + p->second + ", " + b + ")";
+            if (const auto* p = product(b)) return "__fma_rn(" + p->first + ", " + p->second + ", " + a + ")";
+            return "ag::rn_add(" + a + ", " + b + ")";
+        }
         return L.contract ? "(" + a + " + " + b + ")" : "ag::rn_add(" + a + ", " + b + ")";
     }
     std::string sub(const std::string& a, const std::string& b) const {
         if (dfm) return NS + "sub(" + a + ", " + b + ")";
+        if (xfma) {
+            if (const auto* p = product(a)) return "__fma_rn(" + p->first + ", " + p->second + ", -" + b + ")";
+            if (const auto* p = product(b)) return "__fma_rn(-" + p->first + ", " + p->second + ", " + a + ")";
+            return "ag::rn_sub(" + a + ", " + b + ")";
+        }
         return L.contract ? "(" + a + " - " + b + ")" : "ag::rn_sub(" + a + ", " + b + ")";
     }
     // Products and quotients inside composite nodes carry the range check
@@ -511,13 +546,24 @@ struct Gen {
     std::string mul(const std::string& a, const std::string& b) const {
         if (dfm && (zero_vars.count(a) || zero_vars.count(b))) return NS + "mul(" + a + ", " + b + ")";
         if (dfm) return NS + "ck(" + NS + "mul(" + a + ", " + b + "), " + cur_ok + ")";
+        if (xfma) {
+            const std::string v = "ag::rn_mul(" + a + ", " + b + ")";
+            prods[v] = {a, b};
+            return v;
+        }
         return L.contract ? "(" + a + " * " + b + ")" : "ag::rn_mul(" + a + ", " + b + ")";
     }
     std::string div(const std::string& a, const std::string& b) const {
         if (dfm) return NS + "ck(" + NS + "div(" + a + ", " + b + "), " + cur_ok + ")";
         return "ag::rn_div(" + a + ", " + b + ")";
     }
-    std::string neg(const std::string& a) const { return dfm ? NS + "neg(" + a + ")" : "(-" + a + ")"; }
+    std::string neg(const std::string& a) const {
+        if (dfm) return NS + "neg(" + a + ")";
+        const std::string v = "(-" + a + ")";
+        if (xfma)
+            if (const auto* p = product(a)) prods[v] = {"(-" + p->first + ")", p->second};
+        return v;
+    }
     std::string lit(double v) const {
         if (tfm) return tf_literal(v);
         if (dfm) return NS + "dfc(" + hexlit(v) + ")";
@@ -569,6 +615,8 @@ struct Gen {
         for (size_t c = 0; c < exprs.size(); ++c) {
             const std::string nm = pre + std::to_string(id) + "_" + std::to_string(c);
             o << "        const " << (is_bool ? "bool" : W) << " " << nm << " = " << exprs[c] << ";\n";
+            if (xfma)
+                if (const auto* p = product(exprs[c])) prods[nm] = std::make_pair(p->first, p->second);
             names.push_back(nm);
         }
         val[size_t(id)] = names;
@@ -1023,10 +1071,12 @@ std::string generate_source(const Plan& plan_in, const Lowering& low, const std:
     std::ostringstream o;
     if (!chunk_only) {
         o << "// generated by aether_gb300 from an aether-ir/1 plan\n";
+        const bool f64n = emu || P.dst_dtype == DType::F64;   // some lane runs native FP64 code
+        if (f64n && native_needs_tf(P)) o << "#define AG_NATIVE_TF 1\n";
         o << "#include \"ag_device.cuh\"\n";
         if (low.math >= 1) o << "#include \"ag_emu64.cuh\"\n";
-        if (tfx) o << "#include \"ag_tf64.cuh\"\n";
-        if (tfx && uses_trig(P)) o << "#include \"ag_tf64_trig.cuh\"\n";
+        if (tfx || (f64n && native_needs_tf(P))) o << "#include \"ag_tf64.cuh\"\n";
+        if ((tfx || f64n) && (uses_trig(P) || draws_normals(P))) o << "#include \"ag_tf64_trig.cuh\"\n";
         if (low.math >= 1 && draws_normals(P)) o << "#include \"ag_emu64_bm.cuh\"\n";
         o << "#define AG_BLOCK " << low.block << "\n#define AG_IPT " << low.ipt << "\n#define AG_VEC " << vec << "\n";
     }
@@ -1250,18 +1300,21 @@ std::string generate_batch_source(const std::vector<const Plan*>& plans, const s
     bool emu = false;
     for (const Lowering& l : lows) emu = emu || l.math >= 1;
     o << "// generated by aether_gb300: batch of " << plans.size() << " plans\n";
+    bool bm = false, tf = false, tft = false, ntf = false;
+    for (size_t p = 0; p < plans.size(); ++p) {
+        const Plan& P = *plans[p];
+        const bool f64n = lows[p].math >= 1 || P.dst_dtype == DType::F64, tfx = lows[p].math == 3 && P.dst_dtype == DType::F64;
+        bm = bm || (lows[p].math >= 1 && draws_normals(P));
+        tf = tf || tfx;
+        ntf = ntf || (f64n && native_needs_tf(P));
+        tft = tft || (f64n && (uses_trig(P) || draws_normals(P)));
+    }
+    if (ntf) o << "#define AG_NATIVE_TF 1\n";
     o << "#include \"ag_device.cuh\"\n";
     if (emu) o << "#include \"ag_emu64.cuh\"\n";
-    bool bm = false;
-    for (size_t p = 0; p < plans.size(); ++p) bm = bm || (lows[p].math >= 1 && draws_normals(*plans[p]));
-    if (bm) o << "#include \"ag_emu64_bm.cuh\"\n";
-    bool tf = false;
-    for (size_t p = 0; p < plans.size(); ++p) tf = tf || (lows[p].math == 3 && plans[p]->dst_dtype == DType::F64);
-    if (tf) o << "#include \"ag_tf64.cuh\"\n";
-    bool tft = false;
-    for (size_t p = 0; p < plans.size(); ++p)
-        tft = tft || (lows[p].math == 3 && plans[p]->dst_dtype == DType::F64 && uses_trig(*plans[p]));
+    if (tf || ntf) o << "#include \"ag_tf64.cuh\"\n";
     if (tft) o << "#include \"ag_tf64_trig.cuh\"\n";
+    if (bm) o << "#include \"ag_emu64_bm.cuh\"\n";
     o << "#define AG_BLOCK " << block << "\n#define AG_IPT " << ipt << "\n";
     std::vector<int> vecs;
     for (size_t p = 0; p < plans.size(); ++p) {

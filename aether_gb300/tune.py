@@ -41,20 +41,16 @@ def _device_name():
     return torch.cuda.get_device_name(torch.cuda.current_device())
 
 
-# Device headers only FP64-grade (math 3) kernels include.
-_TF_HEADERS = ("ag_tf64.cuh", "ag_tf64_tables.cuh", "ag_tf64_trig.cuh", "ag_tf64_trig_tables.cuh")
-
-
 def _code_digest(math=0):
-    """Digest of the device runtime a generated kernel of this lowering can
-    include (the payload headers under their bare names; the consumer headers
-    under aether/ never reach a generated kernel, and the triple-float headers
-    only reach math-3 kernels): a tuning result stays valid only for the code
-    it was measured on."""
+    """Digest of the device runtime a generated kernel can include (the payload
+    headers under their bare names; the consumer headers under aether/ never
+    reach a generated kernel; native code takes its FP64 functions from the
+    triple-float headers): a tuning result stays valid only for the code it was
+    measured on."""
     from . import rtc
     h = hashlib.sha1()
     for name, src in sorted(rtc.payload().headers.items()):
-        if name.startswith("aether/") or (name in _TF_HEADERS and math != 3):
+        if name.startswith("aether/"):
             continue
         h.update(name.encode())
         h.update(src)

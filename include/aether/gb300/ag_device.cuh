@@ -70,8 +70,15 @@ __device__ __forceinline__ q4 philox_block(ag_u64 seed, ag_u32 global, ag_u32 co
 // Word -> real conversions (Backend.h:123-157). Each is an exact scaling plus
 // at most one rounding, spelled with explicit round-to-nearest operations so
 // no contraction can change them.
+// w 2^-32 + 2^-33 = (2 w + 1) 2^-33 is exact in a double, so its bits are put
+// together in integers: the leading one of 2 w + 1 gives the exponent, the
+// bits below it the fraction. (The conversion, product and sum it replaces run
+// on the FP64 pipe, three of the four operations there of a uniform draw.)
+// Shifts by 32 leave 0.
 __device__ __forceinline__ double u01_f64(ag_u32 w) {
-    return __dadd_rn(__dmul_rn((double)w, 2.3283064365386963e-10), 1.1641532182693481e-10);
+    const unsigned lz = (unsigned)__clz((int)w);   // 32 for w = 0
+    const ag_u32 f = __funnelshift_lc(0u, w, lz + 1u) | __funnelshift_lc(0u, 1u, lz);
+    return __hiloint2double((int)(((1022u - lz) << 20) | (f >> 12)), (int)(f << 20));
 }
 __device__ __forceinline__ float u01_f32(ag_u32 w) {
     return __fmul_rn((float)(((w >> 9) << 1) | 1u), 5.9604645e-8f);
@@ -93,10 +100,25 @@ __device__ __forceinline__ double u01hq_f64(ag_u32 x, ag_u32 y) {
 // and its FP64 library functions; rsqrt is 1/sqrt(x) with both steps correctly
 // rounded, the host spelling of math/root.h:64-76, so it is bit-exact with the
 // reference's CPU path. Float: the full-precision float functions.
+// Generated plans define AG_NATIVE_TF where they call one of the guarded
+// double functions, and take these from ag_tf64.cuh and ag_tf64_trig.cuh.
 // ---------------------------------------------------------------------------
+#ifndef AG_NATIVE_TF
 __device__ __forceinline__ double f_sqrt(double x) { return __dsqrt_rn(x); }
-__device__ __forceinline__ float f_sqrt(float x) { return __fsqrt_rn(x); }
 __device__ __forceinline__ double f_rsqrt(double x) { return __ddiv_rn(1.0, __dsqrt_rn(x)); }
+__device__ __forceinline__ double f_exp(double x) { return exp(x); }
+__device__ __forceinline__ double f_log(double x) { return log(x); }
+__device__ __forceinline__ double f_log1p(double x) { return log1p(x); }
+__device__ __forceinline__ double f_sin(double x) { return sin(x); }
+__device__ __forceinline__ double f_cos(double x) { return cos(x); }
+__device__ __forceinline__ double rn_div(double a, double b) { return __ddiv_rn(a, b); }
+#endif
+__device__ __forceinline__ float f_exp(float x) { return expf(x); }
+__device__ __forceinline__ float f_log(float x) { return logf(x); }
+__device__ __forceinline__ float f_log1p(float x) { return log1pf(x); }
+__device__ __forceinline__ float f_sin(float x) { return sinf(x); }
+__device__ __forceinline__ float f_cos(float x) { return cosf(x); }
+__device__ __forceinline__ float f_sqrt(float x) { return __fsqrt_rn(x); }
 __device__ __forceinline__ float f_rsqrt(float x) { return __fdiv_rn(1.0f, __fsqrt_rn(x)); }
 __device__ __forceinline__ double f_abs(double x) { return fabs(x); }
 __device__ __forceinline__ float f_abs(float x) { return fabsf(x); }
@@ -108,15 +130,10 @@ __device__ __forceinline__ float f_neg(float x) { return -x; }
 #define AG_UNARY(NAME, DFN, FFN)                                              \
     __device__ __forceinline__ double f_##NAME(double x) { return DFN(x); } \
     __device__ __forceinline__ float f_##NAME(float x) { return FFN(x); }
-AG_UNARY(exp, exp, expf)
 AG_UNARY(expm1, expm1, expm1f)
 AG_UNARY(exp2, exp2, exp2f)
-AG_UNARY(log, log, logf)
-AG_UNARY(log1p, log1p, log1pf)
 AG_UNARY(log2, log2, log2f)
 AG_UNARY(log10, log10, log10f)
-AG_UNARY(sin, sin, sinf)
-AG_UNARY(cos, cos, cosf)
 AG_UNARY(tan, tan, tanf)
 AG_UNARY(asin, asin, asinf)
 AG_UNARY(acos, acos, acosf)
@@ -146,7 +163,6 @@ AG_BINARY(hypot, hypot, hypotf)
 __device__ __forceinline__ double rn_add(double a, double b) { return __dadd_rn(a, b); }
 __device__ __forceinline__ double rn_sub(double a, double b) { return __dsub_rn(a, b); }
 __device__ __forceinline__ double rn_mul(double a, double b) { return __dmul_rn(a, b); }
-__device__ __forceinline__ double rn_div(double a, double b) { return __ddiv_rn(a, b); }
 __device__ __forceinline__ float rn_add(float a, float b) { return __fadd_rn(a, b); }
 __device__ __forceinline__ float rn_sub(float a, float b) { return __fsub_rn(a, b); }
 __device__ __forceinline__ float rn_mul(float a, float b) { return __fmul_rn(a, b); }
@@ -180,7 +196,9 @@ __device__ __forceinline__ double draw01(double*, ag_u64 seed, ag_u32 g, ag_u32 
 __device__ __forceinline__ float draw01(float*, ag_u64 seed, ag_u32 g, ag_u32 c) {
     return u01_f32(philox_block(seed, g, c).x);
 }
+#ifndef AG_NATIVE_TF
 __device__ __forceinline__ double drawn(double*, ag_u64 seed, ag_u32 g, ag_u32 c) { return normal_f64(seed, g, c); }
+#endif
 __device__ __forceinline__ float drawn(float*, ag_u64 seed, ag_u32 g, ag_u32 c) { return normal_f32(seed, g, c); }
 
 // ---------------------------------------------------------------------------

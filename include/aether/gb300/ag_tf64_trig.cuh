@@ -93,4 +93,82 @@ __device__ __forceinline__ tf sin_(tf x, bool& ok) { return trig_(x, false, ok);
 __device__ __forceinline__ tf cos_(tf x, bool& ok) { return trig_(x, true, ok); }
 
 }  // namespace t64
+
+#if defined(__CUDACC__) || defined(__CUDACC_RTC__) || defined(AG_N64_HOST_CHECK)
+namespace n64 {
+#if defined(__CUDACC__) || defined(__CUDACC_RTC__)
+__device__ AG_N64_NOINLINE double slow_sin(double x) { return ::sin(x); }
+__device__ AG_N64_NOINLINE double slow_cos(double x) { return ::cos(x); }
+__device__ AG_N64_NOINLINE double slow_normal(ag_u64 seed, ag_u32 g, ag_u32 c) { return ag::normal_f64(seed, g, c); }
+#endif
+// Below 2^-27, sin x = x and cos x = 1 to a quarter of an ulp.
+__device__ __forceinline__ double sin(double x) {
+    bool ok = true;
+    const tf a = t64::from_double_ck(x, ok);
+    const double r = join(t64::sin_(a, ok));
+    if (((unsigned)__double2hiint(x) & 0x7fffffffu) < (996u << 20)) return x;
+    return ok ? r : slow_sin(x);
+}
+__device__ __forceinline__ double cos(double x) {
+    bool ok = true;
+    const tf a = t64::from_double_ck(x, ok);
+    const double r = join(t64::cos_(a, ok));
+    if (((unsigned)__double2hiint(x) & 0x7fffffffu) < (996u << 20)) return 1.0;
+    return ok ? r : slow_cos(x);
+}
+
+// The Box-Muller draw of ag::normal_f64 step by step: u and v are the
+// reference's doubles, built in integers; log u, sqrt(-2 log u) and sin(pi v)
+// are each rounded to a double as there, and two FP64 products are left of
+// about 120 FP64 operations.
+__device__ __forceinline__ double normal(ag_u64 seed, ag_u32 g, ag_u32 c) {
+    const ag::q4 x = ag::philox_block(seed, g, c);
+    // u = z 2^-53 + 2^-54 rounded to a double = w 2^-54, w < 2^54: exact below
+    // 1/2, to even above it. Split in 24 + 23 + 7 bits from the leading one.
+    const ag_u64 z = (ag_u64)x.x ^ ((ag_u64)x.y << 21);
+    const ag_u64 w = z < (1ull << 52) ? 2ull * z + 1ull : 2ull * (z + (z & 1ull));
+    const ag_u32 wh = (ag_u32)(w >> 32), wl = (ag_u32)w;
+    const int lz = __clz((int)wh) - 10;   // -1 where u is 1
+    bool ok = wh != 0u && lz >= 0;
+    const ag_u32 nh = __funnelshift_l(wl, wh, (unsigned)lz), nl = wl << (lz & 31);
+    const ag_u32 top = __funnelshift_l(nl, nh, 2u);   // bits 53..30
+    const float my = __fsub_rn(__int_as_float((int)(0x4B000000u | ((nl >> 7) & 0x7fffffu))), 8388608.0f);
+    const float mz = __fsub_rn(__int_as_float((int)(0x4B000000u | (nl & 127u))), 8388608.0f);
+    const tf u = t64::mk3(__int_as_float((int)(((ag_u32)(126 - lz) << 23) | (top & 0x7fffffu))),
+                          __fmul_rn(my, __int_as_float((int)((ag_u32)(80 - lz) << 23))),
+                          __fmul_rn(mz, __int_as_float((int)((ag_u32)(73 - lz) << 23))));
+    const double l = join(t64::log_s<false, t64::LOG_S0>(0.0f, u));   // < 0
+    const double m2l = __hiloint2double((int)(((unsigned)__double2hiint(l) & 0x7fffffffu) + (1u << 20)), __double2loint(l));
+    const double s = join(t64::sqrt_pos_(t64::from_double_ck(m2l, ok)));
+    // v = zy 2^-52 + 2^-53 rounded = V 2^-53, V <= 2^54, its leading bit moved to bit 54
+    const ag_u64 zy = (ag_u64)x.z ^ ((ag_u64)x.w << 21);
+    const ag_u64 V = zy < (1ull << 52) ? 2ull * zy + 1ull : 2ull * (zy + (zy & 1ull));
+    const ag_u32 vh = (ag_u32)(V >> 32), vl = (ag_u32)V;
+    const int lv = __clz((int)vh) - 9;
+    ok = ok && vh != 0u;
+    const ag_u32 mh = __funnelshift_l(vl, vh, (unsigned)lv), ml = vl << (lv & 31);
+    const double v = __hiloint2double((int)(((ag_u32)(1024 - lv) << 20) | ((mh >> 2) & 0xfffffu)),
+                                      (int)((mh << 30) | (ml >> 2)));
+    const tf p = t64::from_double_ck(__dmul_rn(v, 3.1415926535897932), ok);
+    const double sv = join(t64::sin_(p, ok));
+    const double r = __dmul_rn(s, sv);
+    return ok ? r : slow_normal(seed, g, c);
+}
+}  // namespace n64
+
+namespace t64 {
+// N(0, 1) leaves of FP64-grade plans: the reference's formula, as in the
+// native lowering, bit for bit.
+template <bool U = false>
+__device__ __forceinline__ tf normal_df(ag_u64 seed, ag_u32 g, ag_u32 c) {
+    return dfc(n64::normal(seed, g, c));
+}
+}  // namespace t64
+#endif
+
+#ifdef AG_NATIVE_TF
+__device__ __forceinline__ double f_sin(double x) { return n64::sin(x); }
+__device__ __forceinline__ double f_cos(double x) { return n64::cos(x); }
+__device__ __forceinline__ double drawn(double*, ag_u64 seed, ag_u32 g, ag_u32 c) { return n64::normal(seed, g, c); }
+#endif
 }  // namespace ag
