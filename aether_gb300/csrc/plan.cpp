@@ -1331,24 +1331,23 @@ std::string generate_batch_source(const std::vector<const Plan*>& plans, const s
     o << "extern \"C\" __global__ void __launch_bounds__(AG_BLOCK"
       << (min_blocks > 0 ? ", " + std::to_string(min_blocks) : std::string()) << ") " << base
       << "(const AgItem* __restrict__ items, int n_items, ag_u64 total_tiles) {\n";
-    o << "    __shared__ int s_item;\n";
-    o << "    for (ag_u64 t = blockIdx.x; t < total_tiles; t += gridDim.x) {\n";
-    o << "        if (threadIdx.x == 0) {\n";
-    o << "            int lo = 0, hi = n_items - 1;\n";
-    o << "            while (lo < hi) {\n";
-    o << "                const int mid = (lo + hi + 1) >> 1;\n";
-    o << "                if (items[mid].tile0 <= t) lo = mid; else hi = mid - 1;\n";
-    o << "            }\n";
-    o << "            s_item = lo;\n";
-    o << "        }\n";
-    o << "        __syncthreads();\n";
-    o << "        const AgItem& it = items[s_item];\n";
-    o << "        __syncthreads();\n";
+    // Every warp finds its tile's item itself (ag::next_item), the loads for it
+    // issued a tile ahead. A binary search by one thread with two barriers a
+    // tile stood still: 2048 uneven arrays took 1014 us, this 870.
+    o << "    ag_u64 t = blockIdx.x;\n";
+    o << "    if (t >= total_tiles) return;\n";
+    o << "    int cur = ag::item_at(items, n_items, 0, t);\n";
+    o << "    for (;;) {\n";
+    o << "        const ag_u64 probe = ag::probe_items(items, n_items, cur);\n";
+    o << "        const AgItem& it = items[cur];\n";
     o << "        const ag_u64 ch = t - it.tile0;\n";
     o << "        switch (it.plan) {\n";
     for (size_t p = 0; p < plans.size(); ++p)
         o << "        case " << p << ": ag_chunk_p" << p << "<" << vecs[p] << ">(it.a, ch); break;\n";
-    o << "        default: break;\n        }\n    }\n}\n";
+    o << "        default: break;\n        }\n";
+    o << "        t += gridDim.x;\n";
+    o << "        if (t >= total_tiles) return;\n";
+    o << "        cur = ag::next_item(items, n_items, cur, probe, t);\n    }\n}\n";
     return o.str();
 }
 

@@ -411,6 +411,38 @@ __device__ __forceinline__ void butterfly32(T& h, T& c) {
 
 namespace ag {
 
+// The last item of a work list whose first tile is at most t, known to be `lo`
+// or later (items[lo].tile0 <= t). One warp probes 32 items a step, so a list
+// of thousands takes two or three dependent loads where a binary search takes
+// eleven or more. All lanes of the warp call it with the same arguments.
+template <class Item>
+__device__ __forceinline__ int item_at(const Item* __restrict__ items, int n_items, int lo, ag_u64 t) {
+    const int lane = threadIdx.x & 31;
+    int hi = n_items - 1;
+    while (lo < hi) {
+        const int step = (hi - lo + 31) / 32;
+        const int p = lo + step * (lane + 1);
+        const int k = __popc(__ballot_sync(0xffffffffu, p <= hi && items[p].tile0 <= t));
+        lo += step * k;
+        hi = min(hi, lo + step - 1);
+    }
+    return lo;
+}
+// First tile of the item `lane + 1` places after `cur`; beyond the list, none.
+template <class Item>
+__device__ __forceinline__ ag_u64 probe_items(const Item* __restrict__ items, int n_items, int cur) {
+    const int p = cur + 1 + (int)(threadIdx.x & 31);
+    return p < n_items ? items[p].tile0 : ~0ull;
+}
+// The same as item_at from `cur`, given probe_items(items, n_items, cur) read
+// before the previous tile's work, which hides the load: the next tile of a
+// CTA is rarely more than 32 items on.
+template <class Item>
+__device__ __forceinline__ int next_item(const Item* __restrict__ items, int n_items, int cur, ag_u64 probe, ag_u64 t) {
+    const int k = __popc(__ballot_sync(0xffffffffu, probe <= t));
+    return k < 32 ? cur + k : item_at(items, n_items, cur + 32, t);
+}
+
 // Finish a CTA's share of a sum plan: reduce its threads' (hi, comp) pairs with
 // the warp butterfly and a fixed cross-warp order, publish the CTA's partial,
 // and let the CTA that arrives last combine all partials in a fixed order (so
