@@ -418,6 +418,7 @@ struct Gen {
     std::ostringstream body;  // per-lane code
     bool dfm = false;         // double-float working type (emulated FP64)
     bool tfm = false;         // with dfm: triple-float working type (FP64-grade, math 3)
+    bool pm = false;          // every value holds two samples (f32x2 arithmetic, ag_emu64.cuh)
     std::string NS = "ag::e64::";   // namespace of the working type's functions
     std::string pre = "t";    // variable prefix
     bool direct = false;      // leaves load their own sample `s` (per-lane fallback function)
@@ -453,14 +454,23 @@ struct Gen {
     }
 
     Gen(const Plan& p, const Lowering& l, const std::vector<int>& c, bool df_mode = false, std::string prefix = "t",
-        bool force_double = false, bool tf_mode = false)
+        bool force_double = false, bool tf_mode = false, bool pairs = false)
         : P(p), L(l), ctx(c), val(p.nodes.size()), done(p.nodes.size(), 0), dfm(df_mode || tf_mode), tfm(tf_mode),
-          pre(std::move(prefix)) {
-        NS = tfm ? "ag::t64::" : "ag::e64::";
+          pm(pairs), pre(std::move(prefix)) {
+        NS = pm ? (tfm ? "ag::y64::" : "ag::x64::") : tfm ? "ag::t64::" : "ag::e64::";
         if (tfm) kSafeLo = -80;
         W = tfm ? "ag::t64::tf" : dfm ? "ag::e64::df" : ((P.dst_dtype == DType::F64 || force_double) ? "double" : "float");
         S = P.dst_dtype == DType::F64 ? "double" : "float";
         xfma = W == "double" && L.contract && native_needs_tf(P);
+        W1 = W;
+        if (pm) W = tfm ? "ag::t64::tf2" : dfm ? "ag::e64::df2" : "ag::d2";
+    }
+    std::string W1;   // one sample's working type
+    // A value every sample shares.
+    std::string shared(const std::string& v) const { return pm ? (dfm ? NS : std::string("ag::")) + "both(" + v + ")" : v; }
+    std::string pick(const std::string& c, const std::string& a, const std::string& b) const {
+        if (pm) return (dfm ? NS : std::string("ag::")) + "sel(" + c + ", " + a + ", " + b + ")";
+        return "(" + c + " ? " + a + " : " + b + ")";
     }
 
     // Contraction in native code that calls ag::n64, written out: those
@@ -518,8 +528,8 @@ struct Gen {
     std::string add(const std::string& a, const std::string& b) const {
         if (dfm) return NS + "add(" + a + ", " + b + ")";
         if (xfma) {
-            if (const auto* p = product(a)) return "__fma_rn(" + p->first + ", " + p->second + ", " + b + ")";
-            if (const auto* p = product(b)) return "__fma_rn(" + p->first + ", " + p->second + ", " + a + ")";
+            if (const auto* p = product(a)) return "ag::rn_fma(" + p->first + ", " + p->second + ", " + b + ")";
+            if (const auto* p = product(b)) return "ag::rn_fma(" + p->first + ", " + p->second + ", " + a + ")";
             return "ag::rn_add(" + a + ", " + b + ")";
         }
         return L.contract ? "(" + a + " + " + b + ")" : "ag::rn_add(" + a + ", " + b + ")";
@@ -527,8 +537,8 @@ struct Gen {
     std::string sub(const std::string& a, const std::string& b) const {
         if (dfm) return NS + "sub(" + a + ", " + b + ")";
         if (xfma) {
-            if (const auto* p = product(a)) return "__fma_rn(" + p->first + ", " + p->second + ", -" + b + ")";
-            if (const auto* p = product(b)) return "__fma_rn(-" + p->first + ", " + p->second + ", " + a + ")";
+            if (const auto* p = product(a)) return "ag::rn_fma(" + p->first + ", " + p->second + ", ag::rn_neg(" + b + "))";
+            if (const auto* p = product(b)) return "ag::rn_fma(ag::rn_neg(" + p->first + "), " + p->second + ", " + a + ")";
             return "ag::rn_sub(" + a + ", " + b + ")";
         }
         return L.contract ? "(" + a + " - " + b + ")" : "ag::rn_sub(" + a + ", " + b + ")";
@@ -559,15 +569,16 @@ struct Gen {
     }
     std::string neg(const std::string& a) const {
         if (dfm) return NS + "neg(" + a + ")";
-        const std::string v = "(-" + a + ")";
+        if (!xfma && !pm) return "(-" + a + ")";
+        const std::string v = "ag::rn_neg(" + a + ")";
         if (xfma)
-            if (const auto* p = product(a)) prods[v] = {"(-" + p->first + ")", p->second};
+            if (const auto* p = product(a)) prods[v] = {"ag::rn_neg(" + p->first + ")", p->second};
         return v;
     }
     std::string lit(double v) const {
-        if (tfm) return tf_literal(v);
-        if (dfm) return NS + "dfc(" + hexlit(v) + ")";
-        return "((" + W + ")" + hexlit(v) + ")";
+        if (tfm) return shared(tf_literal(v));
+        if (dfm) return shared(NS + "dfc(" + hexlit(v) + ")");
+        return shared("((" + W1 + ")" + hexlit(v) + ")");
     }
     // A literal as three floats split here, exactly for every normal double
     // (no FP64 work in the kernel).
@@ -594,16 +605,18 @@ struct Gen {
     std::string call(const std::string& name, const std::vector<std::string>& args, int id) const {
         std::string a;
         for (size_t i = 0; i < args.size(); ++i) a += (i ? ", " : "") + args[i];
-        if (!dfm) return "ag::f_" + name + "(" + a + ")";
+        if (!dfm) return (pm ? "ag::f2_" : "ag::f_") + name + "(" + a + ")";
         static const std::set<std::string> own = {"sqrt", "rsqrt", "log", "log1p", "abs", "sign", "min", "max"};
         if (name == "sin" || name == "cos" || name == "exp") return NS + "" + name + "_(" + a + ", " + okv(id) + ")";
         if (name == "log1p" && abs_of_input(P.nodes[size_t(id)].kids[0]))
             return NS + "log1p_nn_(" + a + ")";   // |input| is >= 0 and within the input range check
-        if (own.count(name)) return NS + "" + name + "_(" + a + ")";
+        // those with a plain double-float form have their template under _t
+        static const std::set<std::string> t = {"sqrt", "rsqrt", "log", "log1p"};
+        if (own.count(name)) return NS + name + (pm && !tfm && t.count(name) ? "_t(" : "_(") + a + ")";
         return NS + "nat_" + name + "(" + a + ")";
     }
     std::string gtx(const std::string& a, const std::string& b) const {
-        return dfm ? NS + "gt(" + a + ", " + b + ")" : "(" + a + " > " + b + ")";
+        return dfm ? NS + "gt(" + a + ", " + b + ")" : pm ? "ag::gt(" + a + ", " + b + ")" : "(" + a + " > " + b + ")";
     }
 
     std::ostringstream& out_for(int id) { return ctx[size_t(id)] ? pro : body; }
@@ -614,7 +627,7 @@ struct Gen {
         std::vector<std::string> names;
         for (size_t c = 0; c < exprs.size(); ++c) {
             const std::string nm = pre + std::to_string(id) + "_" + std::to_string(c);
-            o << "        const " << (is_bool ? "bool" : W) << " " << nm << " = " << exprs[c] << ";\n";
+            o << "        const " << (is_bool ? (pm ? "ag::e64::b2" : "bool") : W) << " " << nm << " = " << exprs[c] << ";\n";
             if (xfma)
                 if (const auto* p = product(exprs[c])) prods[nm] = std::make_pair(p->first, p->second);
             names.push_back(nm);
@@ -692,7 +705,7 @@ struct Gen {
             kids_safe = m > kOpenLo && 2 * m >= kSafeLo;
         }
         std::vector<std::string> e;
-        const std::string gid = c0 ? "g0" : "g";
+        const std::string gid = c0 ? "g0" : pm ? "g, h" : "g";
         const std::string sid = pre + std::to_string(id);
 
         if (op == "in") {
@@ -703,13 +716,18 @@ struct Gen {
                 if (direct)
                     src = "((const " + ctype_of(n.dtype) + "*)a.ops[" + std::to_string(n.k) + "])[(ag_u64)" +
                           std::to_string(c) + " * a.pitch[" + std::to_string(n.k) + "] + " + (c0 ? "0" : "s") + "]";
+                // the next sample's source: lane l + 1 of the thread
+                const std::string src1 = "in" + std::to_string(n.k) + "[" + std::to_string(c) + "][l + 1]";
+                const std::string f0 = pm ? "ag::e64::pk(0.0f, 0.0f)" : "0.0f";
                 if (pbool) {
                     e.push_back("(" + src + " != 0)");
                 } else if (dfm && n.dtype == DType::F32) {
-                    e.push_back(tfm ? "ag::t64::mk3((float)" + src + ", 0.0f, 0.0f)"
-                                    : NS + "mk((float)" + src + ", 0.0f)");   // exact
+                    const std::string x = pm ? "ag::e64::pk((float)" + src + ", (float)" + src1 + ")" : "(float)" + src;
+                    e.push_back(tfm ? "ag::t64::mk3(" + x + ", " + f0 + ", " + f0 + ")" : NS + "mk(" + x + ", " + f0 + ")");   // exact
                 } else if (dfm) {
-                    e.push_back(NS + "from_double_ck((double)" + src + ", " + okv(id) + ")");
+                    e.push_back(NS + "from_double_ck((double)" + src + (pm ? ", (double)" + src1 : "") + ", " + okv(id) + ")");
+                } else if (pm) {
+                    e.push_back("ag::d2{(double)" + src + ", (double)" + src1 + "}");
                 } else {
                     e.push_back("(" + W + ")" + src);
                 }
@@ -718,7 +736,7 @@ struct Gen {
         } else if (op == "sc") {
             const std::string s = "a.sc[" + std::to_string(n.k) + "]";
             const std::string k = std::to_string(n.k);
-            def(id, {tfm ? "ag::t64::dfc(" + s + ")" : dfm ? NS + "mk(a.sch[" + k + "], a.scl[" + k + "])" : "(" + W + ")" + s});
+            def(id, {shared(tfm ? "ag::t64::dfc(" + s + ")" : dfm ? NS + "mk(a.sch[" + k + "], a.scl[" + k + "])" : "(" + W1 + ")" + s)});
         } else if (op == "lit") {
             def(id, {lit(n.lit)});
             if (n.lit == 0.0) zero_vars.insert(val[size_t(id)][0]);   // products with it are exact zeros
@@ -770,6 +788,7 @@ struct Gen {
             for (int c = 0; c < n.comps; ++c) {
                 const std::string a = V(0)[size_t(c)], b = V(1)[size_t(c)];
                 if (dfm && !logical && !K(0).is_bool) e.push_back(NS + "" + op + "(" + a + ", " + b + ")");
+                else if (pm) e.push_back("ag::" + op + "(" + a + ", " + b + ")");
                 else e.push_back("(" + a + " " + sym.at(op) + " " + b + ")");
             }
             def(id, e, true);
@@ -779,7 +798,7 @@ struct Gen {
         } else if (op == "select") {   // Elementwise.h:809-846
             const bool per_sample = K(0).shape.empty();
             for (int c = 0; c < n.comps; ++c)
-                e.push_back("(" + V(0)[per_sample ? 0 : size_t(c)] + " ? " + V(1)[size_t(c)] + " : " + V(2)[size_t(c)] + ")");
+                e.push_back(pick(V(0)[per_sample ? 0 : size_t(c)], V(1)[size_t(c)], V(2)[size_t(c)]));
             def(id, e, n.is_bool);
         } else if (op == "comp") {
             val[size_t(id)] = {V(0)[size_t(n.k)]};
@@ -859,7 +878,7 @@ struct Gen {
             auto q = [&](const std::string& num) { return dfm ? mul(num, rd) : div(num, d); };
             if (dim == 2) {
                 o << "        const " << W << " " << d << " = " << sub(mulkk(m[0], m[3]), mulkk(m[1], m[2])) << ";\n";
-                if (dfm && op == "inv") o << "        const " << W << " " << rd << " = " << NS << "recip(" << d << ");\n";
+                if (dfm && op == "inv") o << "        const " << W << " " << rd << " = " << NS << (pm && !tfm ? "recip_t(" : "recip(") << d << ");\n";
                 if (op == "det") e = {d};
                 else e = {q(m[3]), q(neg(m[1])), q(neg(m[2])), q(m[0])};
             } else {
@@ -869,7 +888,7 @@ struct Gen {
                   << add(sub(mul(a, sub(mulkk(ee, k), mulkk(f, h))), mul(b, sub(mulkk(dd, k), mulkk(f, g)))),
                          mul(c, sub(mulkk(dd, h), mulkk(ee, g))))
                   << ";\n";
-                if (dfm && op == "inv") o << "        const " << W << " " << rd << " = " << NS << "recip(" << d << ");\n";
+                if (dfm && op == "inv") o << "        const " << W << " " << rd << " = " << NS << (pm && !tfm ? "recip_t(" : "recip(") << d << ");\n";
                 if (op == "det") {
                     e = {d};
                 } else {
@@ -922,7 +941,7 @@ struct Gen {
             std::string acc = term(0);
             for (int c = 1; c < m; ++c) {
                 const std::string t = term(c);
-                acc = op == "maxnorm" ? "(" + gtx(t, acc) + " ? (" + t + ") : (" + acc + "))" : add(t, acc);
+                acc = op == "maxnorm" ? pick(gtx(t, acc), "(" + t + ")", "(" + acc + ")") : add(t, acc);
             }
             if (op == "norm") acc = call("sqrt", {acc}, id);
             if (op == "rnorm") acc = div(lit(1.0), call("sqrt", {acc}, id));
@@ -931,7 +950,7 @@ struct Gen {
             const std::string key = "a.key[" + std::to_string(n.k) + "]";
             const bool b0 = K(0).shape.empty();
             const bool b1 = n.kids.size() > 1 && K(1).shape.empty();
-            const std::string wp = "(" + W + "*)0";
+            const std::string wp = "(" + W1 + "*)0";
             // N(0, 1) with literal parameters: 0 + 1 z is z bit for bit (z != 0)
             const bool std01 = n.kids.size() > 1 && K(0).op == "lit" && K(0).lit == 0.0 && K(1).op == "lit" &&
                                K(1).lit == 1.0;
@@ -960,8 +979,9 @@ struct Gen {
                     e.push_back(div(neg(call("log", {u01("AG_SALT_EXPONENTIAL", cc)}, id)), x0));
                 } else {   // DistributionLeaf.h:380-385
                     const std::string u = u01("AG_SALT_BERNOULLI", cc);
-                    e.push_back("(" + (dfm ? NS + "lt(" + u + ", " + x0 + ")" : "(" + u + " < " + x0 + ")") + " ? " +
-                                lit(1.0) + " : " + lit(0.0) + ")");
+                    const std::string less = dfm ? NS + "lt(" + u + ", " + x0 + ")"
+                                             : pm ? "ag::lt(" + u + ", " + x0 + ")" : "(" + u + " < " + x0 + ")";
+                    e.push_back(pick(less, lit(1.0), lit(0.0)));
                 }
             }
             def(id, e);
@@ -1019,6 +1039,27 @@ bool uses_trig(const Plan& P) {
     return false;
 }
 
+// Trees with a logarithm, an exponential, a sine or cosine, or a normal draw:
+// 65 to 200 FP32-pipe operations in double-float for each.
+bool heavy(const Plan& P) {
+    static const std::set<std::string> ops = {"exp", "log", "log1p", "sin", "cos", "normal", "lognormal", "exponential"};
+    for (const Node& n : P.nodes)
+        if (ops.count(n.op)) return true;
+    return false;
+}
+
+// Whether a tree can be generated two samples at a time: any of numbers, with
+// comparisons only as conditions of a selection between numbers.
+bool pairable(const Plan& P) {
+    for (const Node& n : P.nodes) {
+        if (n.op == "at0" || n.op == "and" || n.op == "or" || n.op == "not") return false;
+        if (n.op == "in" && n.is_bool) return false;
+        if (n.op == "select" && n.is_bool) return false;
+        if (cmp_ops().count(n.op) && P.nodes[size_t(n.kids[0])].is_bool) return false;
+    }
+    return true;
+}
+
 // Plans with normal or lognormal leaves include the Box-Muller header when
 // lowered to double-float.
 bool draws_normals(const Plan& P) {
@@ -1059,7 +1100,14 @@ std::string generate_source(const Plan& plan_in, const Lowering& low, const std:
     if (dst_ff && !prec) fail("ff destinations are written by the precision form (math = 2)");
     Gen g(P, low, ctx, emu, emu ? "d" : "t", false, tfx);
     g.root_to_double = emu && P.dst_dtype == DType::F64;
-    const std::vector<std::string> root = g.emit(P.root);
+    g.emit(P.root);
+    // The same tree two samples at a time, for the lane counts it divides: the
+    // FP32-pipe arithmetic of the emulated lowerings and of ag::n64 takes one
+    // issue slot and half the code for both (ag_emu64.cuh).
+    const bool pairs = (emu || (P.dst_dtype == DType::F64 && native_needs_tf(P))) && pairable(P);
+    Gen gp(P, low, ctx, emu, "q", false, tfx, pairs);
+    gp.root_to_double = g.root_to_double;
+    if (pairs) gp.emit(P.root);
     Lowering nat = low;
     nat.math = 0;
     Gen gn(P, nat, ctx, false, "n", true);
@@ -1150,24 +1198,66 @@ std::string generate_source(const Plan& plan_in, const Lowering& low, const std:
     if (defer) o << "    unsigned bad_ = 0u;\n";
     o << g.pro.str();
     if (store) o << "    " << S << " out[" << OC << "][L];\n";
-    o << "#pragma unroll\n    for (int l = 0; l < L; ++l) {\n";
-    if (P.has_random) o << "        const ag_u32 g = a.offset + (ag_u32)(s0[l / VEC] + (ag_u64)(l % VEC));\n";
-    if (emu) o << "        bool ok_ = ok0_;\n";
-    o << g.body.str();
-    // Final working values of the output components. The output range test
-    // is left out when the magnitude bounds of the root keep every value of a
-    // lane that passed its other checks inside [2^-88, 2^126).
+    // Reassembly of a double-float: on the FP64 pipe (two conversions and an
+    // addition, 50 clocks a warp) where a function of 65 FP32-pipe operations
+    // or more per element hides it, in integers (out_double) elsewhere.
+    // Measured, FP64 pipe and integers: the large streaming expression over
+    // 2^26 x 3 1506 and 1593 us, N(0, 1) draws 593 and 625 us for 2^26; a + b c
+    // over 2^23 x 3 152 and 125 us, 3x3 inverses 421 and 273 us. A
+    // triple-float's five operations are never hidden (stream 959 and 861 us
+    // for 2^24 x 3, inverses 753 and 457 us).
+    const std::string to_dbl = tfx || (!prec && !heavy(P)) ? "out_double(" : "to_double(";
+    // The output range test is left out when the magnitude bounds of the root
+    // keep every value of a lane that passed its other checks inside [2^-88,
+    // 2^126), and a NaN (the root of a negative number) stays one: a float
+    // pair's, or one reassembled on the FP64 pipe. In integers it would not.
+    auto out_safe = [&](Gen& G) {
+        return emu && to_dbl == "to_double(" && G.lo_of(P.root) >= -88 && G.hi_of(P.root) <= 125;
+    };
+    // One lane loop: the values of each sample, then what is done with them.
+    std::vector<std::string> root;
+    auto lanes_open = [&](Gen& G) {
+        o << "#pragma unroll\n    for (int l" << (G.pm ? "p = 0; lp < L; lp += 2" : " = 0; l < L; ++l") << ") {\n";
+        if (G.pm) o << "        const int l = lp;\n";
+        if (P.has_random) o << "        const ag_u32 g = a.offset + (ag_u32)(s0[l / VEC] + (ag_u64)(l % VEC));\n";
+        if (P.has_random && G.pm)
+            o << "        const ag_u32 h = a.offset + (ag_u32)(s0[(l + 1) / VEC] + (ag_u64)((l + 1) % VEC));\n";
+        if (emu) o << (G.pm ? "        ag::e64::b2 ok_ = {true, true};\n" : "        bool ok_ = ok0_;\n");
+        o << G.body.str();
+        root = G.val[size_t(P.root)];
+        if (!G.pm) return;
+        // from here on one sample at a time
+        const bool dbl = emu && !prec;   // the values leave as doubles
+        const std::string fn = G.dfm ? "ag::e64::ln" : "ag::ln", T1 = dbl ? "double" : G.W1;
+        if (dbl && !out_safe(G))
+            for (int c = 0; c < P.dst_comps; ++c) o << "        " << G.NS << "out_double_ok(" << root[size_t(c)] << ", ok_);\n";
+        if (emu) o << "        const ag::e64::b2 okp_ = ok_;\n";
+        for (int c = 0; c < P.dst_comps; ++c) {
+            const std::string n = std::to_string(c), r = root[size_t(c)];
+            if (dbl) o << "        const ag::e64::d2 rd" << n << " = " << G.NS << to_dbl << r << ");\n";
+            o << "        const " << T1 << " ra" << n << " = " << (dbl ? "rd" + n + ".a" : fn + "0(" + r + ")") << ", rb" << n << " = "
+              << (dbl ? "rd" + n + ".b" : fn + "1(" + r + ")") << ";\n";
+            root[size_t(c)] = "r" + n;
+        }
+        o << "#pragma unroll\n        for (int k_ = 0; k_ < 2; ++k_) {\n        const int l = lp + k_;\n";
+        if (emu) o << "        bool ok_ = k_ ? okp_.b : okp_.a;\n";
+        for (int c = 0; c < P.dst_comps; ++c)
+            o << "        const " << T1 << " r" << c << " = k_ ? rb" << c << " : ra" << c << ";\n";
+    };
     const std::string FW = emu ? "double" : W;
-    const bool out_safe = emu && g.lo_of(P.root) >= (tfx ? -80 : -88) && g.hi_of(P.root) <= 125;
+    auto lanes_close = [&](Gen& G) {
+    // Final working values of the output components.
     for (int c = 0; c < P.dst_comps; ++c) {
         if (prec) {
             o << "        ag::e64::df fv" << c << " = " << root[size_t(c)] << ";\n";
-            if (!out_safe) o << "        ok_ = ok_ && ag::e64::out_ok(fv" << c << ");\n";
+            if (!out_safe(G)) o << "        ok_ = ok_ && ag::e64::out_ok(fv" << c << ");\n";
+        } else if (emu && G.pm) {
+            o << "        double fv" << c << " = " << root[size_t(c)] << ";\n";
         } else if (emu) {
-            o << "        double fv" << c << " = " << g.NS << "to_double(" << root[size_t(c)] << ");\n";
-            if (!out_safe) o << "        ok_ = ok_ && " << g.NS << "out_ok(" << root[size_t(c)] << ");\n";
+            o << "        double fv" << c << " = " << G.NS << to_dbl << root[size_t(c)] << ");\n";
+            if (!out_safe(G)) o << "        " << G.NS << "out_double_ok(" << root[size_t(c)] << ", ok_);\n";
         } else {
-            o << "        const " << W << " fv" << c << " = " << root[size_t(c)] << ";\n";
+            o << "        const " << G.W1 << " fv" << c << " = " << root[size_t(c)] << ";\n";
         }
     }
     if (defer) {
@@ -1228,7 +1318,17 @@ std::string generate_source(const Plan& plan_in, const Lowering& low, const std:
         if (prec) o << "acc = ag::e64::add(acc, fv0);\n";   // per-thread float-float sum
         else o << "ag::neumaier_add(acc_h, acc_c, (double)fv0);\n";
     }
-    o << "    }\n";
+    o << (G.pm ? "    }\n    }\n" : "    }\n");
+    };
+    if (pairs) {
+        o << "    if constexpr (L % 2 == 0) {\n";
+        lanes_open(gp);
+        lanes_close(gp);
+        o << "    } else {\n";
+    }
+    lanes_open(g);
+    lanes_close(g);
+    if (pairs) o << "    }\n";
     if (store) {
         o << "    " << S << "* __restrict__ po = (" << S << "*)a.dst;\n";
         o << "    if (full_) {\n#pragma unroll\n    for (int c = 0; c < " << OC << "; ++c)\n#pragma unroll\n        for (int j = 0; j < AG_IPT; ++j) ag::vec_io<VEC, " << S

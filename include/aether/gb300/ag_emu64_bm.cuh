@@ -59,34 +59,40 @@ __device__ __forceinline__ df from_u54_2m54(ag_u64 w, ag_u32 sgn) {
 // r^2/24). C r = (pi C) t and C r^3 = (pi C) t r^2, so only the float r of the
 // small terms needs pi; the leading product is (pi C) t in double-float.
 // |S| >= sin(pi/4096) >= |C r| except where S = 0: the sum is led by S.
-__device__ __forceinline__ df sin_from_period_table(const f4& sc, df t) {
-    const float th = t.hi;
+template <class F>
+__device__ __forceinline__ dfT<F> sin_from_period_table(dfT<F> S, dfT<F> PC, dfT<F> t) {
+    const F th = t.hi;
     // r = pi t rounded once (pi's and t's low parts joined by FMA): the
     // quadratic term needs r to float accuracy
-    const float rh = __fmaf_rn(AG_PI_HI, th, __fmaf_rn(AG_PI_HI, t.lo, __fmul_rn(AG_PI_LO, th)));
-    const float rh2 = __fmul_rn(rh, rh);
-    const float cub = __fmul_rn(__fmul_rn(th, rh2), __fmaf_rn(rh2, 8.33333333e-3f, -1.66666667e-1f));
-    const float cm1 = __fmul_rn(rh2, __fmaf_rn(rh2, 4.16666667e-2f, -0.5f));
-    const df S = mk(sc.x, sc.y), PC = mk(sc.z, sc.w);
-    return add_quick(add_quick(S, mul_u(PC, t)), __fmaf_rn(S.hi, cm1, __fmul_rn(PC.hi, cub)));
+    const F rh = ffma(bc<F>(AG_PI_HI), th, ffma(bc<F>(AG_PI_HI), t.lo, fmul(bc<F>(AG_PI_LO), th)));
+    const F rh2 = fmul(rh, rh);
+    const F cub = fmul(fmul(th, rh2), ffma(rh2, bc<F>(8.33333333e-3f), bc<F>(-1.66666667e-1f)));
+    const F cm1 = fmul(rh2, ffma(rh2, bc<F>(4.16666667e-2f), bc<F>(-0.5f)));
+    return add_quick(add_quick(S, mul_u(PC, t)), ffma(S.hi, cm1, fmul(PC.hi, cub)));
 }
 
-// U: the product is left unnormalised (the draw is only reassembled into a double)
-template <bool U = false>
-__device__ __forceinline__ df normal_df(ag_u64 seed, ag_u32 g, ag_u32 c) {
+// The integer part of one draw.
+struct bm_words {
+    float s;        // log(u) = log(s + w)
+    df w;
+    float fh, fl;   // the remainder of v, in units of 2^-35 and 2^-53 half-turns
+    f4 sc;          // (S, pi C) of v's table point
+};
+__device__ __forceinline__ bm_words bm_draw(ag_u64 seed, ag_u32 g, ag_u32 c) {
     const ag::q4 x = ag::philox_block(seed, g, c);
+    bm_words b;
     // u is the reference's double z 2^-53 + 2^-54 (random/detail/Backend.h
     // uniformDoubleHq): exact below 1/2, rounded to even above it, where it is
     // k 2^-53 with k = z + (z & 1). So u = w 2^-54 with w = 2 z + 1 below 1/2,
     // and 1 - u = w 2^-54 with w = 2^54 - 2 k (even, at most 2^53) above it.
-    const ag_u64 z = (ag_u64)x.x ^ ((ag_u64)x.y << 21);
-    const bool lower = z < (1ull << 52);
-    const ag_u64 w = lower ? 2ull * z + 1ull : (1ull << 54) - 2ull * (z + (z & 1ull));
     // log(u) for u in [2^-54, 1/2) or log1p(-w) for w in [0, 1/2]; w = 0 (u
     // rounded to 1) gives a zero argument to the square root below, whose NaN
     // sends the lane to the native path
-    const df L = log_s<false, LOG_SRT>(lower ? 0.0f : 1.0f, from_u54_2m54(w, lower ? 0u : 0x80000000u));
-    const df sv = sqrt_pos_(scale(L, -2.0f));   // log u < 0: the argument is positive
+    const ag_u64 z = (ag_u64)x.x ^ ((ag_u64)x.y << 21);
+    const bool lower = z < (1ull << 52);
+    const ag_u64 w = lower ? 2ull * z + 1ull : (1ull << 54) - 2ull * (z + (z & 1ull));
+    b.s = lower ? 0.0f : 1.0f;
+    b.w = from_u54_2m54(w, lower ? 0u : 0x80000000u);
     // v is the reference's double zy 2^-52 + 2^-53: exact below 1, rounded to
     // even above it. So v = V 2^-53 with V = 2 zy + 1, or 2 (zy + (zy & 1))
     // for zy >= 2^52, V <= 2^54. In integers: K = round(V / 2^41) in [0, 8192]
@@ -102,11 +108,32 @@ __device__ __forceinline__ df normal_df(ag_u64 seed, ag_u32 g, ag_u32 c) {
     // both made exact floats by exponent tricks (no conversion unit): Rh as
     // (1.5 2^23 + Rh) - 1.5 2^23, Rl as (2^23 + Rl) - 2^23
     const int Rh = (int)((rh << 14) | (vl >> 18));
-    const float fh = __fsub_rn(__int_as_float(0x4B400000 + Rh), 12582912.0f);
-    const float fl = __fsub_rn(__int_as_float((int)(0x4B000000u | (vl & 0x3ffffu))), 8388608.0f);
-    const df t = fast_two_sum(__fmul_rn(fh, p2f(-35)), __fmul_rn(fl, p2f(-53)));
-    const df sn = sin_from_period_table(ld4(kSinCosPiPeriod, (int)K), t);
+    b.fh = __int_as_float(0x4B400000 + Rh);
+    b.fl = __int_as_float((int)(0x4B000000u | (vl & 0x3ffffu)));
+    b.sc = ld4(kSinCosPiPeriod, (int)K);
+    return b;
+}
+// U: the product is left unnormalised (the draw is only reassembled into a double)
+template <bool U, class F>
+__device__ __forceinline__ dfT<F> bm_normal(F s, dfT<F> w, F fh, F fl, dfT<F> S, dfT<F> PC) {
+    const dfT<F> L = log_s<false, LOG_SRT>(s, w);
+    const dfT<F> sv = sqrt_pos_(scale(L, bc<F>(-2.0f)));   // log u < 0: the argument is positive
+    const dfT<F> t = fast_two_sum(fmul(fsub(fh, bc<F>(12582912.0f)), bc<F>(2.9103830456733704e-11f)),     // 2^-35
+                                  fmul(fsub(fl, bc<F>(8388608.0f)), bc<F>(1.1102230246251565e-16f)));     // 2^-53
+    const dfT<F> sn = sin_from_period_table(S, PC, t);
     return U ? mul_u(sv, sn) : mul(sv, sn);
+}
+template <bool U = false>
+__device__ __forceinline__ df normal_df(ag_u64 seed, ag_u32 g, ag_u32 c) {
+    const bm_words b = bm_draw(seed, g, c);
+    return bm_normal<U>(b.s, b.w, b.fh, b.fl, mk(b.sc.x, b.sc.y), mk(b.sc.z, b.sc.w));
+}
+// The draws of two samples, g and h.
+template <bool U = false>
+__device__ __forceinline__ df2 normal_df(ag_u64 seed, ag_u32 g, ag_u32 h, ag_u32 c) {
+    const bm_words a = bm_draw(seed, g, c), b = bm_draw(seed, h, c);
+    return bm_normal<U>(pk(a.s, b.s), pair(a.w, b.w), pk(a.fh, b.fh), pk(a.fl, b.fl),
+                        mk(pk(a.sc.x, b.sc.x), pk(a.sc.y, b.sc.y)), mk(pk(a.sc.z, b.sc.z), pk(a.sc.w, b.sc.w)));
 }
 
 }  // namespace e64

@@ -42,27 +42,53 @@
 namespace ag {
 namespace t64 {
 
+using e64::b2;
+using e64::bc;
 using e64::df;
+using e64::dfT;
+using e64::f2;
+using e64::fadd;
 using e64::fast_two_sum;
+using e64::ffma;
+using e64::fmul;
+using e64::fneg;
+using e64::fsub;
+using e64::i2;
+using e64::lanes;
+using e64::ln0;
+using e64::ln1;
 using e64::mk;
+using e64::pk;
 using e64::two_prod;
 using e64::two_sum;
 
-struct tf {
-    float x, y, z;
+// One sample (F = float) or two (F = f2, ag_emu64.cuh).
+template <class F>
+struct tfT {
+    F x, y, z;
 };
+typedef tfT<float> tf;
+typedef tfT<f2> tf2;
 
-__device__ __forceinline__ tf mk3(float x, float y, float z) {
-    tf r;
+template <class F>
+__device__ __forceinline__ tfT<F> mk3(F x, F y, F z) {
+    tfT<F> r;
     r.x = x;
     r.y = y;
     r.z = z;
     return r;
 }
-__device__ __forceinline__ tf from_df(df v) { return mk3(v.hi, v.lo, 0.0f); }
-__device__ __forceinline__ tf neg(tf a) { return mk3(-a.x, -a.y, -a.z); }
-__device__ __forceinline__ tf scale(tf a, float p2) {
-    return mk3(__fmul_rn(a.x, p2), __fmul_rn(a.y, p2), __fmul_rn(a.z, p2));
+__device__ __forceinline__ tf2 pair(tf a, tf b) { return mk3(pk(a.x, b.x), pk(a.y, b.y), pk(a.z, b.z)); }
+__device__ __forceinline__ tf ln0(tf2 v) { return mk3(ln0(v.x), ln0(v.y), ln0(v.z)); }
+__device__ __forceinline__ tf ln1(tf2 v) { return mk3(ln1(v.x), ln1(v.y), ln1(v.z)); }
+__device__ __forceinline__ tf2 both(tf v) { return pair(v, v); }   // a value all samples share
+template <class F>
+__device__ __forceinline__ tfT<F> from_df(dfT<F> v) { return mk3(v.hi, v.lo, bc<F>(0.0f)); }
+template <class F>
+__device__ __forceinline__ tfT<F> neg(tfT<F> a) { return mk3(fneg(a.x), fneg(a.y), fneg(a.z)); }
+template <class F>
+__device__ __forceinline__ tfT<F> scale(tfT<F> a, F p2) {
+    return mk3(fmul(a.x, p2), fmul(a.y, p2), fmul(a.z, p2));
 }
 
 // ---------------------------------------------------------------------------
@@ -72,83 +98,93 @@ __device__ __forceinline__ tf scale(tf a, float p2) {
 // are exact pairs; their errors and the third floats form the third level.
 // Under cancellation the result keeps an absolute error near 2^-71 of the
 // larger operand.
-__device__ __forceinline__ tf add(tf a, tf b) {
-    const df s = two_sum(a.x, b.x);
-    const df t = two_sum(a.y, b.y);
-    const df u = two_sum(s.lo, t.hi);
-    const float z = __fadd_rn(__fadd_rn(t.lo, u.lo), __fadd_rn(a.z, b.z));
-    const df w = two_sum(s.hi, u.hi);
+template <class F>
+__device__ __forceinline__ tfT<F> add(tfT<F> a, tfT<F> b) {
+    const dfT<F> s = two_sum(a.x, b.x);
+    const dfT<F> t = two_sum(a.y, b.y);
+    const dfT<F> u = two_sum(s.lo, t.hi);
+    const F z = fadd(fadd(t.lo, u.lo), fadd(a.z, b.z));
+    const dfT<F> w = two_sum(s.hi, u.hi);
     return mk3(w.hi, w.lo, z);
 }
-__device__ __forceinline__ tf sub(tf a, tf b) { return add(a, neg(b)); }
+template <class F>
+__device__ __forceinline__ tfT<F> sub(tfT<F> a, tfT<F> b) { return add(a, neg(b)); }
 // a + b for operands of one sign: |s.hi| is at least either leading float,
 // so the last combination is a Fast2Sum.
-__device__ __forceinline__ tf add_fast(tf a, tf b) {
-    const df s = two_sum(a.x, b.x);
-    const df t = two_sum(a.y, b.y);
-    const df u = two_sum(s.lo, t.hi);
-    const float z = __fadd_rn(__fadd_rn(t.lo, u.lo), __fadd_rn(a.z, b.z));
-    const df w = fast_two_sum(s.hi, u.hi);
+template <class F>
+__device__ __forceinline__ tfT<F> add_fast(tfT<F> a, tfT<F> b) {
+    const dfT<F> s = two_sum(a.x, b.x);
+    const dfT<F> t = two_sum(a.y, b.y);
+    const dfT<F> u = two_sum(s.lo, t.hi);
+    const F z = fadd(fadd(t.lo, u.lo), fadd(a.z, b.z));
+    const dfT<F> w = fast_two_sum(s.hi, u.hi);
     return mk3(w.hi, w.lo, z);
 }
 // a + b where a leads: |a.x| >= |b.x| (or a.x = 0) and |a + b| >= |a| / 2, so
 // the leading floats join by Fast2Sum and the result cannot cancel.
-__device__ __forceinline__ tf add_lead(tf a, tf b) {
-    const df s = fast_two_sum(a.x, b.x);
-    const df t = two_sum(a.y, b.y);
-    const df u = two_sum(s.lo, t.hi);
-    const float z = __fadd_rn(__fadd_rn(t.lo, u.lo), __fadd_rn(a.z, b.z));
-    const df w = fast_two_sum(s.hi, u.hi);
+template <class F>
+__device__ __forceinline__ tfT<F> add_lead(tfT<F> a, tfT<F> b) {
+    const dfT<F> s = fast_two_sum(a.x, b.x);
+    const dfT<F> t = two_sum(a.y, b.y);
+    const dfT<F> u = two_sum(s.lo, t.hi);
+    const F z = fadd(fadd(t.lo, u.lo), fadd(a.z, b.z));
+    const dfT<F> w = fast_two_sum(s.hi, u.hi);
     return mk3(w.hi, w.lo, z);
 }
 // The reassembly into a double rounds x + y + z once whatever their overlap,
 // so the root of a plan has no cheaper form here.
-__device__ __forceinline__ tf add_fast_u(tf a, tf b) { return add_fast(a, b); }
+template <class F>
+__device__ __forceinline__ tfT<F> add_fast_u(tfT<F> a, tfT<F> b) { return add_fast(a, b); }
 
 // a b: the three products of the first two levels as exact pairs, the
 // third-level products by FMA; the dropped terms are below 2^-70 of the
 // product.
-__device__ __forceinline__ tf mul(tf a, tf b) {
-    const df p = two_prod(a.x, b.x);
-    const df q1 = two_prod(a.x, b.y);
-    const df q2 = two_prod(a.y, b.x);
-    const float r = __fmaf_rn(a.y, b.y, __fmaf_rn(a.x, b.z, __fmul_rn(a.z, b.x)));
-    const df s = two_sum(q1.hi, q2.hi);
-    const df u = two_sum(p.lo, s.hi);
-    const float z = __fadd_rn(__fadd_rn(__fadd_rn(q1.lo, q2.lo), __fadd_rn(s.lo, u.lo)), r);
-    const df w = fast_two_sum(p.hi, u.hi);   // |u.hi| is about 2^-23 |p.hi| at most
+template <class F>
+__device__ __forceinline__ tfT<F> mul(tfT<F> a, tfT<F> b) {
+    const dfT<F> p = two_prod(a.x, b.x);
+    const dfT<F> q1 = two_prod(a.x, b.y);
+    const dfT<F> q2 = two_prod(a.y, b.x);
+    const F r = ffma(a.y, b.y, ffma(a.x, b.z, fmul(a.z, b.x)));
+    const dfT<F> s = two_sum(q1.hi, q2.hi);
+    const dfT<F> u = two_sum(p.lo, s.hi);
+    const F z = fadd(fadd(fadd(q1.lo, q2.lo), fadd(s.lo, u.lo)), r);
+    const dfT<F> w = fast_two_sum(p.hi, u.hi);   // |u.hi| is about 2^-23 |p.hi| at most
     return mk3(w.hi, w.lo, z);
 }
-__device__ __forceinline__ tf mul(tf a, float f) {
-    const df p = two_prod(a.x, f);
-    const df q = two_prod(a.y, f);
-    const df u = two_sum(p.lo, q.hi);
-    const float z = __fmaf_rn(a.z, f, __fadd_rn(q.lo, u.lo));
-    const df w = fast_two_sum(p.hi, u.hi);
+template <class F>
+__device__ __forceinline__ tfT<F> mul(tfT<F> a, F f) {
+    const dfT<F> p = two_prod(a.x, f);
+    const dfT<F> q = two_prod(a.y, f);
+    const dfT<F> u = two_sum(p.lo, q.hi);
+    const F z = ffma(a.z, f, fadd(q.lo, u.lo));
+    const dfT<F> w = fast_two_sum(p.hi, u.hi);
     return mk3(w.hi, w.lo, z);
 }
-__device__ __forceinline__ tf sqr(tf a) {
-    const df p = two_prod(a.x, a.x);
-    const float x2 = __fmul_rn(2.0f, a.x);   // exact
-    const df q = two_prod(x2, a.y);
-    const float r = __fmaf_rn(a.y, a.y, __fmul_rn(x2, a.z));
-    const df u = two_sum(p.lo, q.hi);
-    const float z = __fadd_rn(__fadd_rn(q.lo, u.lo), r);
-    const df w = fast_two_sum(p.hi, u.hi);
+template <class F>
+__device__ __forceinline__ tfT<F> sqr(tfT<F> a) {
+    const dfT<F> p = two_prod(a.x, a.x);
+    const F x2 = fadd(a.x, a.x);   // exact
+    const dfT<F> q = two_prod(x2, a.y);
+    const F r = ffma(a.y, a.y, fmul(x2, a.z));
+    const dfT<F> u = two_sum(p.lo, q.hi);
+    const F z = fadd(fadd(q.lo, u.lo), r);
+    const dfT<F> w = fast_two_sum(p.hi, u.hi);
     return mk3(w.hi, w.lo, z);
 }
 // The square of a double-float as a triple-float (no third input float).
-__device__ __forceinline__ tf sqr_df(df a) {
-    const df p = two_prod(a.hi, a.hi);
-    const df q = two_prod(__fmul_rn(2.0f, a.hi), a.lo);
-    const df u = two_sum(p.lo, q.hi);
-    const float z = __fmaf_rn(a.lo, a.lo, __fadd_rn(q.lo, u.lo));
-    const df w = fast_two_sum(p.hi, u.hi);
+template <class F>
+__device__ __forceinline__ tfT<F> sqr_df(dfT<F> a) {
+    const dfT<F> p = two_prod(a.hi, a.hi);
+    const dfT<F> q = two_prod(fadd(a.hi, a.hi), a.lo);
+    const dfT<F> u = two_sum(p.lo, q.hi);
+    const F z = ffma(a.lo, a.lo, fadd(q.lo, u.lo));
+    const dfT<F> w = fast_two_sum(p.hi, u.hi);
     return mk3(w.hi, w.lo, z);
 }
 // Products read only by sums: the reassembly and every sum above take any
 // overlap, so the same value serves.
-__device__ __forceinline__ tf sqr_u(tf a) { return sqr(a); }
+template <class F>
+__device__ __forceinline__ tfT<F> sqr_u(tfT<F> a) { return sqr(a); }
 
 // Products below 2^-80 in magnitude would push the third float toward the
 // subnormal range; such lanes take the native path.
@@ -157,12 +193,18 @@ __device__ __forceinline__ tf ck(tf v, bool& ok) {
     ok = ok && fabsf(v.x) >= AG_TF_MIN;
     return v;
 }
+__device__ __forceinline__ tf2 ck(tf2 v, b2& ok) {
+    ok.a = ok.a && fabsf(ln0(v.x)) >= AG_TF_MIN;
+    ok.b = ok.b && fabsf(ln1(v.x)) >= AG_TF_MIN;
+    return v;
+}
 
 // (x, y, z) with the overlap of y and z folded into y: y + z as an exact
 // pair, then x with its leading part (two-sums, so x may be the smaller).
-__device__ __forceinline__ tf renorm(tf v) {
-    const df s = two_sum(v.y, v.z);
-    const df w = two_sum(v.x, s.hi);
+template <class F>
+__device__ __forceinline__ tfT<F> renorm(tfT<F> v) {
+    const dfT<F> s = two_sum(v.y, v.z);
+    const dfT<F> w = two_sum(v.x, s.hi);
     return mk3(w.hi, w.lo, s.lo);
 }
 
@@ -170,13 +212,15 @@ __device__ __forceinline__ tf renorm(tf v) {
 // step r' = r + r e, e = 1 - y r. y r is within 2^-46 of 1, so 1 - x of the
 // product is exact (Sterbenz) and its second and third floats join by
 // subtractions that are exact or round at 2^-70.
-__device__ __forceinline__ tf recip(tf y) {
-    const df r = e64::recip(mk(y.x, y.y));
-    const tf m = mul(y, from_df(r));
-    const float e = __fsub_rn(__fsub_rn(__fsub_rn(1.0f, m.x), m.y), m.z);
-    return mk3(r.hi, r.lo, __fmul_rn(r.hi, e));
+template <class F>
+__device__ __forceinline__ tfT<F> recip(tfT<F> y) {
+    const dfT<F> r = e64::recip_t(mk(y.x, y.y));
+    const tfT<F> m = mul(y, from_df(r));
+    const F e = fsub(fsub(fsub(bc<F>(1.0f), m.x), m.y), m.z);
+    return mk3(r.hi, r.lo, fmul(r.hi, e));
 }
-__device__ __forceinline__ tf div(tf a, tf b) { return mul(a, recip(b)); }
+template <class F>
+__device__ __forceinline__ tfT<F> div(tfT<F> a, tfT<F> b) { return mul(a, recip(b)); }
 
 // Comparisons by the sign of the difference: the leading float of a sum
 // carries its sign unless the whole sum is zero at the first two levels.
@@ -190,6 +234,18 @@ __device__ __forceinline__ bool ge(tf a, tf b) { return sgn_(sub(a, b)) >= 0; }
 __device__ __forceinline__ bool le(tf a, tf b) { return sgn_(sub(a, b)) <= 0; }
 __device__ __forceinline__ bool eq(tf a, tf b) { return sgn_(sub(a, b)) == 0; }
 __device__ __forceinline__ bool ne(tf a, tf b) { return sgn_(sub(a, b)) != 0; }
+#define AG_T64_CMP2(NAME) \
+    __device__ __forceinline__ b2 NAME(tf2 x, tf2 y) { return b2{NAME(ln0(x), ln0(y)), NAME(ln1(x), ln1(y))}; }
+AG_T64_CMP2(gt)
+AG_T64_CMP2(lt)
+AG_T64_CMP2(ge)
+AG_T64_CMP2(le)
+AG_T64_CMP2(eq)
+AG_T64_CMP2(ne)
+#undef AG_T64_CMP2
+__device__ __forceinline__ tf2 sel(b2 c, tf2 x, tf2 y) {
+    return pair(c.a ? ln0(x) : ln0(y), c.b ? ln1(x) : ln1(y));
+}
 
 // ---------------------------------------------------------------------------
 // double <-> triple-float.
@@ -214,6 +270,9 @@ __device__ __forceinline__ tf from_double_ck(double v, bool& ok) {
     const float z = __fmul_rn(mz, __int_as_float((int)(se - (52u << 23))));
     return mk3(__int_as_float((int)hb), y, z);
 }
+__device__ __forceinline__ tf2 from_double_ck(double v, double w, b2& ok) {
+    return pair(from_double_ck(v, ok.a), from_double_ck(w, ok.b));
+}
 // Any double (runtime scalars, literals, native results): the split by
 // conversions on the FP64 pipe, exact for normal values.
 __device__ __forceinline__ tf dfc(double v) {
@@ -229,6 +288,7 @@ __device__ __forceinline__ tf dfc(double v) {
 __device__ __forceinline__ double to_double(tf v) {
     return __dadd_rn((double)v.x, __dadd_rn((double)v.y, (double)v.z));
 }
+__device__ __forceinline__ e64::d2 to_double(tf2 v) { return e64::d2{to_double(ln0(v)), to_double(ln1(v))}; }
 __device__ __forceinline__ double as_d(tf v) { return to_double(v); }
 // An output whose three floats were all normal: |x| in [2^-80, 2^127).
 __device__ __forceinline__ bool out_ok(tf v) {
@@ -244,35 +304,39 @@ __device__ __forceinline__ bool out_ok(tf v) {
 // needed to 2^-12 of itself: a.x - s.hi^2 is exact (Sterbenz), and the terms
 // of the second level, each up to 2^-23 a and cancelling to the residual, are
 // summed by two-sums.
-__device__ __forceinline__ tf sqrt_pos_(tf a) {
-    const float y = e64::rsqrt_seed(a.x);
-    const float s0 = __fmul_rn(a.x, y);
-    const df p0 = two_prod(s0, s0);
-    const float r0 = __fadd_rn(__fsub_rn(__fsub_rn(a.x, p0.hi), p0.lo), a.y);
-    const float hy = __fmul_rn(0.5f, y);
-    const df s = fast_two_sum(s0, __fmul_rn(r0, hy));
-    const df P = two_prod(s.hi, s.hi);
-    const df Q = two_prod(__fmul_rn(2.0f, s.hi), s.lo);
-    const df e1 = two_sum(__fsub_rn(a.x, P.hi), a.y);
-    const df e2 = two_sum(e1.hi, -P.lo);
-    const df e3 = two_sum(e2.hi, -Q.hi);
-    const float small = __fsub_rn(__fadd_rn(__fadd_rn(e1.lo, e2.lo), __fadd_rn(e3.lo, a.z)),
-                                  __fmaf_rn(s.lo, s.lo, Q.lo));
-    const float R = __fadd_rn(e3.hi, small);
-    return mk3(s.hi, s.lo, __fmul_rn(R, hy));
+template <class F>
+__device__ __forceinline__ tfT<F> sqrt_pos_(tfT<F> a) {
+    const F y = e64::rsqrt_seed(a.x);
+    const F s0 = fmul(a.x, y);
+    const dfT<F> p0 = two_prod(s0, s0);
+    const F r0 = fadd(fsub(fsub(a.x, p0.hi), p0.lo), a.y);
+    const F hy = fmul(bc<F>(0.5f), y);
+    const dfT<F> s = fast_two_sum(s0, fmul(r0, hy));
+    const dfT<F> P = two_prod(s.hi, s.hi);
+    const dfT<F> Q = two_prod(fadd(s.hi, s.hi), s.lo);
+    const dfT<F> e1 = two_sum(fsub(a.x, P.hi), a.y);
+    const dfT<F> e2 = two_sum(e1.hi, fneg(P.lo));
+    const dfT<F> e3 = two_sum(e2.hi, fneg(Q.hi));
+    const F small = fsub(fadd(fadd(e1.lo, e2.lo), fadd(e3.lo, a.z)),
+                                  ffma(s.lo, s.lo, Q.lo));
+    const F R = fadd(e3.hi, small);
+    return mk3(s.hi, s.lo, fmul(R, hy));
 }
-__device__ __forceinline__ tf sqrt_(tf a) {
-    const tf r = sqrt_pos_(a);
-    return a.x == 0.0f ? mk3(0.0f, 0.0f, 0.0f) : r;
+template <class F>
+__device__ __forceinline__ tfT<F> sqrt_(tfT<F> a) {
+    const tfT<F> r = sqrt_pos_(a);
+    return mk3(e64::or_zero(a.x, r.x), e64::or_zero(a.x, r.y), e64::or_zero(a.x, r.z));
 }
-__device__ __forceinline__ tf sqrt_nn_(tf a) { return sqrt_(a); }
+template <class F>
+__device__ __forceinline__ tfT<F> sqrt_nn_(tfT<F> a) { return sqrt_(a); }
 // a > 0. y = the double-float rsqrt (about 2^-47), then y' = y + y e / 2 with
 // e = 1 - a y^2 formed like the reciprocal's residual.
-__device__ __forceinline__ tf rsqrt_(tf a) {
-    const df y = e64::rsqrt_(mk(a.x, a.y));
-    const tf m = mul(a, sqr_df(y));
-    const float e = __fsub_rn(__fsub_rn(__fsub_rn(1.0f, m.x), m.y), m.z);
-    return mk3(y.hi, y.lo, __fmul_rn(__fmul_rn(y.hi, e), 0.5f));
+template <class F>
+__device__ __forceinline__ tfT<F> rsqrt_(tfT<F> a) {
+    const dfT<F> y = e64::rsqrt_t(mk(a.x, a.y));
+    const tfT<F> m = mul(a, sqr_df(y));
+    const F e = fsub(fsub(fsub(bc<F>(1.0f), m.x), m.y), m.z);
+    return mk3(y.hi, y.lo, fmul(fmul(y.hi, e), bc<F>(0.5f)));
 }
 
 // ---------------------------------------------------------------------------
@@ -283,10 +347,12 @@ __device__ __forceinline__ tf rsqrt_(tf a) {
 // 2^-66 of t). t^2 Q is about 2^-12 of t, so it is formed in double-float
 // (2^-46 of itself, 2^-58 of t) with the coefficient 1/3 as a float pair.
 // ---------------------------------------------------------------------------
-enum { LOG_S0 = 0, LOG_S1 = 1 };
-template <bool checked, int MODE>
-__device__ __forceinline__ tf log_s(float s, tf a) {
-    const float yh = __fadd_rn(s, a.x);
+struct log_row {
+    float A;
+    tf L, E;
+    bool valid;
+};
+__device__ __forceinline__ log_row log_reduce(float yh) {
     const int bits = __float_as_int(yh);
     int e = ((bits >> 23) & 0xff) - 127;
     int mb = (bits & 0x007fffff) | 0x3f800000;
@@ -296,46 +362,79 @@ __device__ __forceinline__ tf log_s(float s, tf a) {
     }
     const float m = __int_as_float(mb);
     const int i = e64::rint_i(__fmaf_rn(m, 1024.0f, -1024.0f)) + AG_TF_LOG_TAB_OFF;
-    const e64::f4 cl = e64::ld4(kLogCL3, i);
-    const float A = __int_as_float((int)((unsigned)__float_as_int(cl.x) - ((unsigned)e << 23)));   // c 2^-e, exact
-    const tf aA = mul(a, A);
-    tf t;
+    const e64::f4 cl = e64::ld4(kLogCL3, i), ep = e64::ld4(kLn2Mul3, e + AG_TF_LN2_TAB_OFF);
+    log_row r;
+    r.A = __int_as_float((int)((unsigned)__float_as_int(cl.x) - ((unsigned)e << 23)));   // c 2^-e, exact
+    r.L = mk3(cl.y, cl.z, cl.w);
+    r.E = mk3(ep.x, ep.y, ep.z);
+    r.valid = yh > 0.0f && e > -120 && e < 120;
+    return r;
+}
+template <class F>
+struct log_rows {
+    F A;
+    tfT<F> L, E;
+    typename lanes<F>::flag valid;
+};
+__device__ __forceinline__ log_rows<float> log_tables(float yh) {
+    const log_row r = log_reduce(yh);
+    return log_rows<float>{r.A, r.L, r.E, r.valid};
+}
+__device__ __forceinline__ log_rows<f2> log_tables(f2 yh) {
+    const log_row r = log_reduce(ln0(yh)), s = log_reduce(ln1(yh));
+    return log_rows<f2>{pk(r.A, s.A), pair(r.L, s.L), pair(r.E, s.E), b2{r.valid, s.valid}};
+}
+__device__ __forceinline__ tf or_nan(bool ok, tf v) { return ok ? v : mk3(__int_as_float(0x7fc00000), 0.0f, 0.0f); }
+__device__ __forceinline__ tf2 or_nan(b2 ok, tf2 v) { return pair(or_nan(ok.a, ln0(v)), or_nan(ok.b, ln1(v))); }
+
+enum { LOG_S0 = 0, LOG_S1 = 1 };
+template <bool checked, int MODE, class F>
+__device__ __forceinline__ tfT<F> log_s(F s, tfT<F> a) {
+    const log_rows<F> R = t64::log_tables(fadd(s, a.x));
+    const tfT<F> aA = mul(a, R.A);
+    tfT<F> t;
     if (MODE == LOG_S0) {
         // a A is within 2^-10 of 1: its leading float less 1 is exact
-        const df d = two_sum(__fsub_rn(aA.x, 1.0f), aA.y);
+        const dfT<F> d = two_sum(fsub(aA.x, bc<F>(1.0f)), aA.y);
         t = mk3(d.hi, d.lo, aA.z);
     } else {
-        const df B = two_sum(A, -1.0f);   // A - 1 exactly
-        t = add(mk3(B.hi, B.lo, 0.0f), aA);
+        const dfT<F> B = two_sum(R.A, bc<F>(-1.0f));   // A - 1 exactly
+        t = add(mk3(B.hi, B.lo, bc<F>(0.0f)), aA);
     }
     // t's third float can be far above an ulp of its second when t is small
     // (a A within 2^-24 of 1 leaves a's third float beside a tiny leading
     // part), and the series below reads t's first two floats only
     t = renorm(t);
     // P = t^2 Q in double-float
-    const float th = t.x;
-    const df tt = mk(t.x, t.y);
-    const float R = __fmaf_rn(th, __fmaf_rn(th, __fmaf_rn(th, 0.142857143f, -0.166666667f), 0.2f), -0.25f);
-    const df G = e64::add_quick(mk(AG_TF_THIRD_HI, AG_TF_THIRD_LO), e64::mul(tt, R));
-    const df Q = e64::add_quick(mk(-0.5f, 0.0f), e64::mul(tt, G));
-    const df P = e64::mul(e64::sqr(tt), Q);
+    const F th = t.x;
+    const dfT<F> tt = mk(t.x, t.y);
+    const F r = ffma(th, ffma(th, ffma(th, bc<F>(0.142857143f), bc<F>(-0.166666667f)), bc<F>(0.2f)), bc<F>(-0.25f));
+    const dfT<F> G = e64::add_quick(mk(bc<F>(AG_TF_THIRD_HI), bc<F>(AG_TF_THIRD_LO)), e64::mul(tt, r));
+    const dfT<F> Q = e64::add_quick(mk(bc<F>(-0.5f), bc<F>(0.0f)), e64::mul(tt, G));
+    const dfT<F> P = e64::mul(e64::sqr(tt), Q);
     // T = t + P: |P| < |t| / 2^11
-    const df h = fast_two_sum(t.x, P.hi);
-    const df k = two_sum(h.lo, t.y);
-    const tf T = mk3(h.hi, k.hi, __fadd_rn(__fadd_rn(k.lo, t.z), P.lo));
+    const dfT<F> h = fast_two_sum(t.x, P.hi);
+    const dfT<F> k = two_sum(h.lo, t.y);
+    const tfT<F> T = mk3(h.hi, k.hi, fadd(fadd(k.lo, t.z), P.lo));
     // e ln2 - log c_i, each from its table as three floats. |e ln2| >= ln2 >
     // 0.29 >= |log c_i| unless e = 0, and |-log c_i| >= 2^-10 >= 2 |T| unless
     // i = 0 (then the leading term is 0): both sums are led by their first term.
-    const e64::f4 ep = e64::ld4(kLn2Mul3, e + AG_TF_LN2_TAB_OFF);
-    const tf res = add_lead(add_lead(mk3(ep.x, ep.y, ep.z), mk3(cl.y, cl.z, cl.w)), T);
-    if (!checked) return res;
-    const bool valid = yh > 0.0f && e > -120 && e < 120;
-    return valid ? res : mk3(__int_as_float(0x7fc00000), 0.0f, 0.0f);
+    const tfT<F> res = add_lead(add_lead(R.E, R.L), T);
+    return checked ? or_nan(R.valid, res) : res;
 }
-__device__ __forceinline__ tf log_(tf a) { return log_s<true, LOG_S0>(0.0f, a); }
-__device__ __forceinline__ tf log1p_(tf a) { return log_s<true, LOG_S1>(1.0f, a); }
+template <class F>
+__device__ __forceinline__ tfT<F> log_(tfT<F> a) {
+    return log_s<true, LOG_S0>(bc<F>(0.0f), a);
+}
+template <class F>
+__device__ __forceinline__ tfT<F> log1p_(tfT<F> a) {
+    return log_s<true, LOG_S1>(bc<F>(1.0f), a);
+}
 // log1p of an argument known to be >= 0 and within the input range
-__device__ __forceinline__ tf log1p_nn_(tf a) { return log_s<false, LOG_S1>(1.0f, a); }
+template <class F>
+__device__ __forceinline__ tfT<F> log1p_nn_(tfT<F> a) {
+    return log_s<false, LOG_S1>(bc<F>(1.0f), a);
+}
 
 // ---------------------------------------------------------------------------
 // Simple nodes, Philox draws and the bridge to native FP64.
@@ -344,9 +443,16 @@ __device__ __forceinline__ tf abs_(tf a) { return sgn_(a) < 0 ? neg(a) : a; }
 __device__ __forceinline__ tf sign_(tf a) { return mk3((float)sgn_(a), 0.0f, 0.0f); }
 __device__ __forceinline__ tf min_(tf a, tf b) { return lt(b, a) ? b : a; }
 __device__ __forceinline__ tf max_(tf a, tf b) { return gt(b, a) ? b : a; }
+__device__ __forceinline__ tf2 abs_(tf2 x) { return pair(abs_(ln0(x)), abs_(ln1(x))); }
+__device__ __forceinline__ tf2 sign_(tf2 x) { return pair(sign_(ln0(x)), sign_(ln1(x))); }
+__device__ __forceinline__ tf2 min_(tf2 x, tf2 y) { return pair(min_(ln0(x), ln0(y)), min_(ln1(x), ln1(y))); }
+__device__ __forceinline__ tf2 max_(tf2 x, tf2 y) { return pair(max_(ln0(x), ln0(y)), max_(ln1(x), ln1(y))); }
 // (2w + 1) 2^-33: exact in the first two floats.
 __device__ __forceinline__ tf draw01_df(ag_u64 seed, ag_u32 g, ag_u32 c) {
     return from_df(e64::draw01_df(seed, g, c));
+}
+__device__ __forceinline__ tf2 draw01_df(ag_u64 seed, ag_u32 g, ag_u32 h, ag_u32 c) {
+    return pair(draw01_df(seed, g, c), draw01_df(seed, h, c));
 }
 // ---------------------------------------------------------------------------
 // exp: x = k ln2/64 + r, |r| <= ln2/128, e^x = 2^(k >> 6) T_(k & 63) (1 + p),
@@ -360,35 +466,43 @@ __device__ __forceinline__ tf draw01_df(ag_u64 seed, ag_u32 g, ag_u32 c) {
 // the result's third float would leave the normal floats (the native lane
 // computes those).
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ tf exp_(tf x, bool& ok) {
-    ok = ok && x.x > -55.0f && x.x < 87.0f;
-    const float kx = __fmul_rn(x.x, AG_TF_INV_LN2_64);
-    const float kf = e64::rint_f(kx);
-    const int k = e64::rint_i(kx);
-    const tf r = renorm(sub(x, mul(mk3(AG_TF_LN2_64_X, AG_TF_LN2_64_Y, AG_TF_LN2_64_Z), kf)));
-    const df rr = mk(r.x, r.y);
-    const float rh = r.x;
-    const float J = __fmaf_rn(rh, __fmaf_rn(rh, 1.98412698e-4f, 1.38888889e-3f), 8.33333333e-3f);
-    const df H = e64::add_quick(mk(AG_TF_24TH_HI, AG_TF_24TH_LO), __fmul_rn(rh, J));
-    const df G = e64::add_quick(mk(AG_TF_SIXTH_HI, AG_TF_SIXTH_LO), e64::mul(rr, H));
-    const df Q = e64::add_quick(mk(0.5f, 0.0f), e64::mul(rr, G));
-    const df P = e64::mul(e64::sqr(rr), Q);
-    // p = r + P: |P| <= r^2 < |r|
-    const df h = fast_two_sum(r.x, P.hi);
-    const df m = two_sum(h.lo, r.y);
-    const tf p = mk3(h.hi, m.hi, __fadd_rn(__fadd_rn(m.lo, r.z), P.lo));
+__device__ __forceinline__ tf exp_table(int k) {
     const e64::f4 tv = e64::ld4(kExp2Tab3, k & 63);
-    const tf T = mk3(tv.x, tv.y, tv.z);
+    return mk3(tv.x, tv.y, tv.z);
+}
+__device__ __forceinline__ tf2 exp_table(i2 k) { return pair(exp_table(k.a), exp_table(k.b)); }
+template <class F>
+__device__ __forceinline__ tfT<F> exp_(tfT<F> x, typename lanes<F>::flag& ok) {
+    e64::within(x.x, -55.0f, 87.0f, ok);
+    const F kx = fmul(x.x, bc<F>(AG_TF_INV_LN2_64));
+    const F kf = e64::rint_f(kx);
+    const typename lanes<F>::whole k = e64::rint_i(kx);
+    const tfT<F> ln2 = mk3(bc<F>(AG_TF_LN2_64_X), bc<F>(AG_TF_LN2_64_Y), bc<F>(AG_TF_LN2_64_Z));
+    const tfT<F> r = renorm(sub(x, mul(ln2, kf)));
+    const dfT<F> rr = mk(r.x, r.y);
+    const F rh = r.x;
+    const F J = ffma(rh, ffma(rh, bc<F>(1.98412698e-4f), bc<F>(1.38888889e-3f)), bc<F>(8.33333333e-3f));
+    const dfT<F> H = e64::add_quick(mk(bc<F>(AG_TF_24TH_HI), bc<F>(AG_TF_24TH_LO)), fmul(rh, J));
+    const dfT<F> G = e64::add_quick(mk(bc<F>(AG_TF_SIXTH_HI), bc<F>(AG_TF_SIXTH_LO)), e64::mul(rr, H));
+    const dfT<F> Q = e64::add_quick(mk(bc<F>(0.5f), bc<F>(0.0f)), e64::mul(rr, G));
+    const dfT<F> P = e64::mul(e64::sqr(rr), Q);
+    // p = r + P: |P| <= r^2 < |r|
+    const dfT<F> h = fast_two_sum(r.x, P.hi);
+    const dfT<F> m = two_sum(h.lo, r.y);
+    const tfT<F> p = mk3(h.hi, m.hi, fadd(fadd(m.lo, r.z), P.lo));
+    const tfT<F> T = t64::exp_table(k);
     // T >= 1 leads T p (|p| < 2^-7)
-    const tf res = add_lead(T, mul(T, p));
-    int e = k >> 6;
-    e = e < -126 ? -126 : (e > 126 ? 126 : e);
-    return scale(res, e64::p2f(e));
+    const tfT<F> res = add_lead(T, mul(T, p));
+    return scale(res, e64::p2f(e64::exp_power(k)));
 }
 #define AG_T64_NATIVE1(NAME)                                                                   \
-    __device__ __forceinline__ tf nat_##NAME(tf x) { return dfc(ag::f_##NAME(as_d(x))); }
+    __device__ __forceinline__ tf nat_##NAME(tf x) { return dfc(ag::f_##NAME(as_d(x))); }      \
+    __device__ __forceinline__ tf2 nat_##NAME(tf2 x) { return pair(nat_##NAME(ln0(x)), nat_##NAME(ln1(x))); }
 #define AG_T64_NATIVE2(NAME)                                                                   \
-    __device__ __forceinline__ tf nat_##NAME(tf a, tf b) { return dfc(ag::f_##NAME(as_d(a), as_d(b))); }
+    __device__ __forceinline__ tf nat_##NAME(tf a, tf b) { return dfc(ag::f_##NAME(as_d(a), as_d(b))); } \
+    __device__ __forceinline__ tf2 nat_##NAME(tf2 x, tf2 y) {                                  \
+        return pair(nat_##NAME(ln0(x), ln0(y)), nat_##NAME(ln1(x), ln1(y)));                   \
+    }
 AG_T64_NATIVE1(expm1)
 AG_T64_NATIVE1(exp2)
 AG_T64_NATIVE1(log2)
@@ -412,6 +526,7 @@ AG_T64_NATIVE2(hypot)
 #undef AG_T64_NATIVE2
 
 }  // namespace t64
+namespace y64 = t64;   // the spelling of a plan's two-sample code
 
 #if defined(__CUDACC__) || defined(__CUDACC_RTC__) || defined(AG_N64_HOST_CHECK)
 // ---------------------------------------------------------------------------
@@ -450,96 +565,208 @@ __device__ AG_N64_NOINLINE double slow_log(double x) { return ::log(x); }
 __device__ AG_N64_NOINLINE double slow_log1p(double x) { return is_zero(x) ? x : ::log1p(x); }
 #endif
 
+using e64::d2;
+using e64::plus;
+using t64::b2;
+using t64::bc;
+using t64::f2;
+using t64::fadd;
+using t64::fmul;
+using t64::fsub;
+using t64::i2;
+using t64::lanes;
+using t64::ln0;
+using t64::ln1;
+using t64::pk;
+using t64::tfT;
+
+// One double or a pair of them, and the triple-float type of as many.
+__device__ __forceinline__ tf split(double v, bool& ok) { return t64::from_double_ck(v, ok); }
+__device__ __forceinline__ t64::tf2 split(d2 v, b2& ok) { return t64::from_double_ck(v.a, v.b, ok); }
+
+using e64::join_bits;
+using e64::to_int;
 // x + y + z rounded to a double in integers and floats alone: the double of x
 // with (y + z) in its units added to its bits. Needs |x| in [2^-75, 2^100) and
-// |y| within a few ulps of x. Below a power of two the unit halves. `g` is the
-// part of (y + z) that was rounded away plus the integer it was rounded to
-// (`i`): |g - i| near 1/2 is a value near a rounding boundary.
-__device__ __forceinline__ double join(tf v, float& g, int& i) {
-    const unsigned xb = (unsigned)__float_as_int(v.x);
-    const unsigned wb = (unsigned)__float_as_int(__fadd_rn(v.y, v.z));
-    const bool down = (xb & 0x7fffffu) == 0u && (wb & 0x7fffffffu) != 0u && ((wb ^ xb) >> 31) != 0u;
-    // 2^(52 - e), with x's sign, from x's exponent field
-    const unsigned sc = ((down ? 307u : 306u) << 23) - (xb & 0x7f800000u) + (xb & 0x80000000u);
-    const float S = __int_as_float((int)sc);
-    const float Y = __fmul_rn(v.y, S), Z = __fmul_rn(v.z, S);   // exact scalings
-    const int i1 = __float2int_rn(Y);
-    g = __fadd_rn(__fsub_rn(Y, (float)i1), Z);
-    i = __float2int_rn(g);
-    const int off = i1 + i;
-    const ag_i64 b = (ag_i64)(((ag_u64)((xb & 0x80000000u) | (((xb & 0x7fffffffu) >> 3) + (896u << 20))) << 32) | (xb << 29)) + off;
-    return __hiloint2double((int)(b >> 32), (int)b);
+// |y| within a few ulps of x. `g` is the last part of (y + z) before it is
+// rounded to the integer `i`: |g - i| near 1/2 is a value near a boundary.
+template <class F>
+__device__ __forceinline__ auto join(tfT<F> v, F& g, typename lanes<F>::whole& i) {
+    const F S = e64::join_scale(v.x, fadd(v.y, v.z));
+    const F Y = fmul(v.y, S), Z = fmul(v.z, S);   // exact scalings
+    const typename lanes<F>::whole i1 = to_int(Y);
+    g = fadd(fsub(Y, e64::to_f(i1)), Z);
+    i = to_int(g);
+    return join_bits(v.x, plus(i1, i));
 }
-__device__ __forceinline__ double join(tf v) {
-    float g;
-    int i;
+template <class F>
+__device__ __forceinline__ auto join(tfT<F> v) {
+    F g;
+    typename lanes<F>::whole i;
     return join(v, g, i);
 }
 // The same, clearing `ok` within 2^-9 of an ulp of a rounding boundary (the
 // triple-float sqrt, recip and quotient are good to 2^-12 of one).
-__device__ __forceinline__ double join_exact(tf v, bool& ok) {
-    float g;
-    int i;
-    const double r = join(v, g, i);
-    ok = ok && fabsf(__fsub_rn(g, (float)i)) < 0.498046875f;
+template <class F>
+__device__ __forceinline__ auto join_exact(tfT<F> v, typename lanes<F>::flag& ok) {
+    F g;
+    typename lanes<F>::whole i;
+    const auto r = join(v, g, i);
+    e64::within(fsub(g, e64::to_f(i)), -0.498046875f, 0.498046875f, ok);
     return r;
 }
 
-__device__ __forceinline__ double sqrt(double x) {
-    bool ok = true;
-    const tf a = t64::from_double_ck(x, ok);
-    const double r = join_exact(t64::sqrt_pos_(a), ok);
-    return ok && a.x > 0.0f ? r : slow_sqrt(x);
+template <class F>
+__device__ __forceinline__ auto sqrt_core(tfT<F> a, typename lanes<F>::flag& ok) {
+    e64::within(a.x, 0.0f, 3e38f, ok);
+    return join_exact(t64::sqrt_pos_(a), ok);
 }
 // 1 / sqrt(x), each step rounded (the host spelling of math/root.h:64-76)
-__device__ __forceinline__ double rsqrt(double x) {
-    bool ok = true;
-    const tf a = t64::from_double_ck(x, ok);
-    const double s = join_exact(t64::sqrt_pos_(a), ok);
-    const double r = join_exact(t64::recip(t64::from_double_ck(s, ok)), ok);
-    return ok && a.x > 0.0f ? r : slow_rsqrt(x);
+template <class F>
+__device__ __forceinline__ auto rsqrt_core(tfT<F> a, typename lanes<F>::flag& ok) {
+    const auto s = sqrt_core(a, ok);
+    return join_exact(t64::recip(split(s, ok)), ok);
 }
-__device__ __forceinline__ double div(double a, double b) {
-    bool ok = true;
-    const tf x = t64::from_double_ck(a, ok), y = t64::from_double_ck(b, ok);
-    const tf q = t64::mul(x, t64::recip(y));
-    const unsigned e = ((unsigned)__float_as_int(q.x) >> 23) & 0xffu;
-    ok = ok && e - 62u <= 160u;   // |q| in [2^-65, 2^96)
-    const double r = join_exact(q, ok);
-    return ok ? r : slow_div(a, b);
+template <class F>
+__device__ __forceinline__ auto div_core(tfT<F> x, tfT<F> y, typename lanes<F>::flag& ok) {
+    const tfT<F> q = t64::mul(x, t64::recip(y));
+    e64::within(e64::fabs_(q.x), 2.7105054e-20f, 7.9228163e28f, ok);   // |q| in (2^-65, 2^96)
+    return join_exact(q, ok);
 }
-__device__ __forceinline__ double exp(double x) {
-    bool ok = true;
-    const tf a = t64::from_double_ck(x, ok);
-    ok = ok && a.x > -50.0f;
-    const double r = join(t64::exp_(a, ok));
-    return ok ? r : slow_exp(x);
+template <class F>
+__device__ __forceinline__ auto exp_core(tfT<F> a, typename lanes<F>::flag& ok) {
+    e64::within(a.x, -50.0f, 3e38f, ok);
+    return join(t64::exp_(a, ok));
 }
-__device__ __forceinline__ double log(double x) {
-    bool ok = true;
-    const tf a = t64::from_double_ck(x, ok);
-    const tf l = t64::log_s<false, t64::LOG_S0>(0.0f, a);
-    ok = ok && a.x > 0.0f && l.x != 0.0f;   // log 1 = 0 has no leading float
-    const double r = join(l);
-    return ok ? r : slow_log(x);
+template <class F>
+__device__ __forceinline__ auto log_core(tfT<F> a, typename lanes<F>::flag& ok) {
+    const tfT<F> l = t64::log_s<false, t64::LOG_S0>(bc<F>(0.0f), a);
+    e64::within(a.x, 0.0f, 3e38f, ok);
+    e64::within(e64::fabs_(l.x), 0.0f, 3e38f, ok);   // log 1 = 0 has no leading float
+    return join(l);
 }
-__device__ __forceinline__ double log1p(double x) {
+template <class F>
+__device__ __forceinline__ auto log1p_core(tfT<F> a, typename lanes<F>::flag& ok) {
+    e64::within(a.x, -0.75f, 3e38f, ok);   // nearer to -1 the reduced argument cancels
+    return join(t64::log_s<false, t64::LOG_S1>(bc<F>(1.0f), a));
+}
+#define AG_N64_FUNCTION(NAME)                                              \
+    __device__ __forceinline__ double NAME(double x) {                     \
+        bool ok = true;                                                    \
+        const tf a = split(x, ok);                                         \
+        const double r = NAME##_core(a, ok);                               \
+        return ok ? r : slow_##NAME(x);                                    \
+    }                                                                      \
+    __device__ __forceinline__ d2 NAME(d2 x) {                             \
+        b2 ok{true, true};                                                 \
+        const t64::tf2 a = split(x, ok);                                   \
+        d2 r = NAME##_core(a, ok);                                         \
+        if (!(ok.a && ok.b)) {                                             \
+            if (!ok.a) r.a = slow_##NAME(x.a);                             \
+            if (!ok.b) r.b = slow_##NAME(x.b);                             \
+        }                                                                  \
+        return r;                                                          \
+    }
+AG_N64_FUNCTION(sqrt)
+AG_N64_FUNCTION(rsqrt)
+AG_N64_FUNCTION(exp)
+AG_N64_FUNCTION(log)
+AG_N64_FUNCTION(log1p)
+__device__ __forceinline__ double div(double x, double y) {
     bool ok = true;
-    const tf a = t64::from_double_ck(x, ok);
-    ok = ok && a.x > -0.75f;   // nearer to -1 the reduced argument cancels
-    const double r = join(t64::log_s<false, t64::LOG_S1>(1.0f, a));
-    return ok ? r : slow_log1p(x);
+    const tf a = split(x, ok), b = split(y, ok);
+    const double r = div_core(a, b, ok);
+    return ok ? r : slow_div(x, y);
+}
+__device__ __forceinline__ d2 div(d2 x, d2 y) {
+    b2 ok{true, true};
+    const t64::tf2 a = split(x, ok), b = split(y, ok);
+    d2 r = div_core(a, b, ok);
+    if (!(ok.a && ok.b)) {
+        if (!ok.a) r.a = slow_div(x.a, y.a);
+        if (!ok.b) r.b = slow_div(x.b, y.b);
+    }
+    return r;
 }
 }  // namespace n64
+
+namespace t64 {
+// A plan's output: x + y + z rounded once, without the FP64 pipe (five
+// operations of it in to_double).
+template <class F>
+__device__ __forceinline__ auto out_double(tfT<F> v) {
+    return n64::join(v);
+}
+template <class F>
+__device__ __forceinline__ void out_double_ok(tfT<F> v, typename lanes<F>::flag& ok) {
+    e64::out_range(v.x, ok);
+}
+}  // namespace t64
 #endif
 
 #ifdef AG_NATIVE_TF
-__device__ __forceinline__ double f_sqrt(double x) { return n64::sqrt(x); }
-__device__ __forceinline__ double f_rsqrt(double x) { return n64::rsqrt(x); }
-__device__ __forceinline__ double f_exp(double x) { return n64::exp(x); }
-__device__ __forceinline__ double f_log(double x) { return n64::log(x); }
-__device__ __forceinline__ double f_log1p(double x) { return n64::log1p(x); }
-__device__ __forceinline__ double rn_div(double a, double b) { return n64::div(a, b); }
+// The functions and operations of native plans, for one sample and for two.
+using e64::b2;
+using e64::both;
+using e64::d2;
+__device__ __forceinline__ d2 rn_add(d2 x, d2 y) { return d2{rn_add(x.a, y.a), rn_add(x.b, y.b)}; }
+__device__ __forceinline__ d2 rn_sub(d2 x, d2 y) { return d2{rn_sub(x.a, y.a), rn_sub(x.b, y.b)}; }
+__device__ __forceinline__ d2 rn_mul(d2 x, d2 y) { return d2{rn_mul(x.a, y.a), rn_mul(x.b, y.b)}; }
+__device__ __forceinline__ double rn_fma(double x, double y, double z) { return __fma_rn(x, y, z); }
+__device__ __forceinline__ d2 rn_fma(d2 x, d2 y, d2 z) { return d2{__fma_rn(x.a, y.a, z.a), __fma_rn(x.b, y.b, z.b)}; }
+__device__ __forceinline__ double rn_neg(double x) { return -x; }
+__device__ __forceinline__ d2 rn_neg(d2 x) { return d2{-x.a, -x.b}; }
+__device__ __forceinline__ double ln0(d2 x) { return x.a; }
+__device__ __forceinline__ double ln1(d2 x) { return x.b; }
+__device__ __forceinline__ d2 sel(b2 c, d2 x, d2 y) { return d2{c.a ? x.a : y.a, c.b ? x.b : y.b}; }
+__device__ __forceinline__ b2 gt(d2 x, d2 y) { return b2{x.a > y.a, x.b > y.b}; }
+__device__ __forceinline__ b2 lt(d2 x, d2 y) { return b2{x.a < y.a, x.b < y.b}; }
+__device__ __forceinline__ b2 ge(d2 x, d2 y) { return b2{x.a >= y.a, x.b >= y.b}; }
+__device__ __forceinline__ b2 le(d2 x, d2 y) { return b2{x.a <= y.a, x.b <= y.b}; }
+__device__ __forceinline__ b2 eq(d2 x, d2 y) { return b2{x.a == y.a, x.b == y.b}; }
+__device__ __forceinline__ b2 ne(d2 x, d2 y) { return b2{x.a != y.a, x.b != y.b}; }
+#define AG_D2_UNARY(NAME) \
+    __device__ __forceinline__ d2 f2_##NAME(d2 x) { return d2{f_##NAME(x.a), f_##NAME(x.b)}; }
+#define AG_D2_BINARY(NAME) \
+    __device__ __forceinline__ d2 f2_##NAME(d2 x, d2 y) { return d2{f_##NAME(x.a, y.a), f_##NAME(x.b, y.b)}; }
+AG_D2_UNARY(abs)
+AG_D2_UNARY(sign)
+AG_D2_UNARY(expm1)
+AG_D2_UNARY(exp2)
+AG_D2_UNARY(log2)
+AG_D2_UNARY(log10)
+AG_D2_UNARY(tan)
+AG_D2_UNARY(asin)
+AG_D2_UNARY(acos)
+AG_D2_UNARY(atan)
+AG_D2_UNARY(tanh)
+AG_D2_UNARY(sinh)
+AG_D2_UNARY(cosh)
+AG_D2_UNARY(floor)
+AG_D2_UNARY(ceil)
+AG_D2_UNARY(trunc)
+AG_D2_UNARY(cbrt)
+AG_D2_UNARY(erf)
+AG_D2_BINARY(pow)
+AG_D2_BINARY(min)
+AG_D2_BINARY(max)
+AG_D2_BINARY(atan2)
+AG_D2_BINARY(hypot)
+#undef AG_D2_UNARY
+#undef AG_D2_BINARY
+#define AG_N64_USE(NAME)                                                              \
+    __device__ __forceinline__ double f_##NAME(double x) { return n64::NAME(x); }     \
+    __device__ __forceinline__ d2 f2_##NAME(d2 x) { return n64::NAME(x); }
+AG_N64_USE(sqrt)
+AG_N64_USE(rsqrt)
+AG_N64_USE(exp)
+AG_N64_USE(log)
+AG_N64_USE(log1p)
+__device__ __forceinline__ double rn_div(double x, double y) { return n64::div(x, y); }
+__device__ __forceinline__ d2 rn_div(d2 x, d2 y) { return n64::div(x, y); }
+__device__ __forceinline__ d2 draw01(double*, ag_u64 seed, ag_u32 g, ag_u32 h, ag_u32 c) {
+    return d2{u01_f64(philox_block(seed, g, c).x), u01_f64(philox_block(seed, h, c).x)};
+}
 #endif
 
 }  // namespace ag

@@ -137,5 +137,35 @@ int main(int argc, char** argv) {
         }
         line("normal", N, worst, 0);
     }
+    {   // the integer reassembly of a double-float against the sum in doubles,
+        // unnormalised pairs and powers of two included; a pair of samples alike
+        long d = 0;
+        for (long i = 0; i < N; ++i) {
+            float hi = (float)(sgn() * logu(-74, 120));
+            if (i % 3 == 0) hi = (float)(sgn() * std::exp2(std::floor(190 * u01(rng) - 70)));
+            float lo = (float)(hi * sgn() * logu(-60, -23));
+            if (i % 5 == 0) lo = 0.0f;
+            const e64::df v = e64::mk(hi, lo), w = e64::mk(-lo * 0.5f + hi, lo);
+            const double want = (double)v.hi + (double)v.lo, want2 = (double)w.hi + (double)w.lo;
+            d += e64::out_double(v) != want;
+            const e64::d2 two = e64::out_double(e64::pair(v, w));
+            d += two.a != want || two.b != want2;
+        }
+        line("reassemble", N, 0, d);
+    }
+    {   // two samples at a time give the same bits as one
+        long d = 0;
+        for (long i = 0; i < N; ++i) {
+            const double x = sgn() * logu(-45, 65), y = sgn() * 4 * u01(rng);
+            auto same = [](double a, double b) { return a == b || (a != a && b != b); };
+#define AG_BOTH(F) { const e64::d2 r = n64::F(e64::d2{x, y}); d += !same(r.a, n64::F(x)) + !same(r.b, n64::F(y)); }
+            AG_BOTH(sqrt) AG_BOTH(rsqrt) AG_BOTH(exp) AG_BOTH(log) AG_BOTH(log1p) AG_BOTH(sin) AG_BOTH(cos)
+            const e64::d2 q = n64::div(e64::d2{x, y}, e64::d2{y, x});
+            d += q.a != n64::div(x, y) || q.b != n64::div(y, x);
+            const e64::d2 z = n64::normal(77, (ag_u32)i, (ag_u32)i + 1u, 2);
+            d += z.a != n64::normal(77, (ag_u32)i, 2) || z.b != n64::normal(77, (ag_u32)i + 1u, 2);
+        }
+        line("pairs", N, 0, d);
+    }
     std::printf("}\n");
 }

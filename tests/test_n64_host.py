@@ -16,7 +16,8 @@ import pytest
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 
-EXACT = ["sqrt", "sqrt_edge", "sqrt_square", "rsqrt", "rsqrt_edge", "div", "div_edge", "div_pairs"]
+EXACT = ["sqrt", "sqrt_edge", "sqrt_square", "rsqrt", "rsqrt_edge", "div", "div_edge", "div_pairs",
+         "reassemble", "pairs"]
 BOUNDS = {"exp": 0.75, "exp_small": 0.75, "log": 0.75, "log_near_1": 0.75, "log1p": 0.75, "log1p_neg": 0.75,
           "log1p_neg_small": 0.75, "sin": 0.75, "sin_unit": 0.75, "sin_small": 0.75, "sin_multiples": 1.0, "cos": 0.75,
           "cos_unit": 0.75, "cos_small": 0.75, "cos_multiples": 1.0}
