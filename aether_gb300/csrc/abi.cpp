@@ -120,20 +120,22 @@ bool capturing(cudaStream_t s) {
 // Plans.
 // ---------------------------------------------------------------------------
 
-ag::Lowering default_lowering(const ag::Plan& p) {
+ag::Lowering default_lowering(const ag::Plan& p, int math) {
     ag::Lowering l;
-    l.block = 256;
+    l.block = ag::default_block(p, math);
+    l.by_size = true;
     l.ipt = 1;
     l.vec = 0;
     l.contract = true;
-    l.math = 0;
-    (void)p;
+    l.math = math;
     return l;
 }
 
 uint64_t ws_needed(const PlanObj& P, uint64_t n) {
     if (!P.plan.wants_sum()) return 0;
-    const uint64_t per = chunk_samples(P, false);   // the scalar kernel has the most chunks
+    // one partial for each of the scalar kernel's chunks at low.block threads, the
+    // most CTAs that plan_shape gives a sum
+    const uint64_t per = uint64_t(P.low.block) * uint64_t(P.low.ipt);
     const uint64_t nch = (n + per - 1) / per;
     return 16 + 16 * std::max<uint64_t>(nch, 1);
 }
@@ -318,9 +320,12 @@ AG_EXPORT int aether_plan_create(const char* ir, const AetherLowering* lowering,
         if (!ir || !out) throw std::runtime_error("plan_create: null argument");
         auto P = std::make_unique<PlanObj>();
         P->plan = ag::parse_plan(ir);
-        P->low = default_lowering(P->plan);
+        P->low = default_lowering(P->plan, lowering && lowering->math >= 0 ? lowering->math : 0);
         if (lowering) {
-            if (lowering->block > 0) P->low.block = lowering->block;
+            if (lowering->block > 0) {
+                P->low.block = lowering->block;
+                P->low.by_size = false;
+            }
             if (lowering->ipt > 0) P->low.ipt = lowering->ipt;
             if (lowering->vec > 0) P->low.vec = lowering->vec;
             if (lowering->contract >= 0) P->low.contract = lowering->contract != 0;
@@ -353,10 +358,13 @@ AG_EXPORT int aether_plan_create(const char* ir, const AetherLowering* lowering,
         cudaFuncAttributes fa{};
         ck(cudaFuncGetAttributes(&fa, reinterpret_cast<const void*>(P->fv)), "cudaFuncGetAttributes");
         P->registers = fa.numRegs;
-        ck(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&P->blocks_per_sm_v, reinterpret_cast<const void*>(P->fv),
-                                                         P->low.block, 0), "occupancy");
-        ck(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&P->blocks_per_sm_s, reinterpret_cast<const void*>(P->fs),
-                                                         P->low.block, 0), "occupancy");
+        for (int i = 0; i < (P->low.by_size ? 4 : 1); ++i) {
+            const int block = P->low.by_size ? std::min(kBlocks[i], P->low.block) : P->low.block;
+            ck(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&P->blocks_per_sm_v[i],
+                                                             reinterpret_cast<const void*>(P->fv), block, 0), "occupancy");
+            ck(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&P->blocks_per_sm_s[i],
+                                                             reinterpret_cast<const void*>(P->fs), block, 0), "occupancy");
+        }
         cudaDeviceGetAttribute(&P->sms, cudaDevAttrMultiProcessorCount, P->dev);
         *out = P.release();
     });
@@ -377,7 +385,9 @@ AG_EXPORT int aether_plan_info(void* plan, AetherPlanInfo* info) {
         info->ipt = P->low.ipt;
         info->vec = P->vec;
         info->registers = P->registers;
-        info->blocks_per_sm = P->blocks_per_sm_v;
+        info->blocks_per_sm = P->blocks_per_sm_v[0];
+        for (int i = 0; P->low.by_size && i < 4; ++i)
+            if (kBlocks[i] <= P->low.block) info->blocks_per_sm = P->blocks_per_sm_v[i];
         info->compile_ms = P->compiled.compile_ms;
     });
 }
@@ -401,6 +411,33 @@ AG_EXPORT int aether_plan_source(void* plan, char* buf, size_t cap, size_t* len)
             buf[n] = '\0';
         }
     });
+}
+
+// Where the caller named no block: the largest that still gives every SM
+// enough CTAs, so that a small launch spreads over the chip. Triple-float
+// kernels (blocks of up to 512) want one per SM: their CTAs run in step through
+// long straight-line code (plain fused expression, 2^24 x 3: 885 us at 512
+// threads, 952 at 256, 975 at 64; 4099 samples: 10.7, 7.3 and 6.5 us). The
+// others want 16 (inverses: 4.9 us at 256 and 3.5 at 64 threads for 4099
+// samples, 41.8 and 39.1 at 128 for 2^20; sums of 65536 terms 14.4 and 11.4 us;
+// from 2^24 samples on all sizes are within 1 %).
+PlanShape plan_shape(const PlanObj& P, uint64_t n, bool vectorized) {
+    const uint64_t lanes = uint64_t(P.low.ipt) * uint64_t(vectorized ? P.vec : 1);
+    int block = P.low.block, i = 0;
+    if (P.low.by_size) {
+        const uint64_t want = (block > 256 ? 1 : 16) * uint64_t(P.sms);
+        for (i = 3; i > 0; --i)
+            if (kBlocks[i] <= P.low.block && (n + kBlocks[i] * lanes - 1) / (kBlocks[i] * lanes) >= want) break;
+        block = kBlocks[i];
+    }
+    uint64_t chunks = (n + uint64_t(block) * lanes - 1) / (uint64_t(block) * lanes);
+    if (P.plan.wants_sum()) {   // no more partials than the workspace of n samples holds
+        const uint64_t per = uint64_t(P.low.block) * uint64_t(P.low.ipt);
+        chunks = std::min(chunks, (n + per - 1) / per);
+    }
+    const int bps = vectorized ? P.blocks_per_sm_v[i] : P.blocks_per_sm_s[i];
+    const uint64_t cap = uint64_t(std::max(bps, 1)) * uint64_t(P.sms);
+    return PlanShape{unsigned(std::max<uint64_t>(1, std::min(chunks, cap))), unsigned(block)};
 }
 
 // Internal (not exported): lets other translation units of the library report
@@ -459,14 +496,9 @@ bool make_args(const PlanObj* P, const AetherLaunch* a, AgArgsHost& k) {
 namespace {
 
 void launch_plan_kernel(const PlanObj& P, AgArgsHost& k, uint64_t n, bool vect, cudaStream_t s) {
-    const uint64_t per = chunk_samples(P, vect);
-    const uint64_t nch = (n + per - 1) / per;
-    const int bps = vect ? P.blocks_per_sm_v : P.blocks_per_sm_s;
-    const uint64_t cap = uint64_t(std::max(bps, 1)) * uint64_t(P.sms);
-    const unsigned grid = unsigned(std::max<uint64_t>(1, std::min(nch, cap)));
+    const PlanShape g = plan_shape(P, n, vect);
     void* params[] = {&k};
-    ck(cudaLaunchKernel(reinterpret_cast<const void*>(vect ? P.fv : P.fs), dim3(grid), dim3(unsigned(P.low.block)),
-                        params, 0, s),
+    ck(cudaLaunchKernel(reinterpret_cast<const void*>(vect ? P.fv : P.fs), dim3(g.grid), dim3(g.block), params, 0, s),
        "cudaLaunchKernel");
 }
 
@@ -753,9 +785,12 @@ AG_EXPORT int aether_plan_generate(const char* ir, const AetherLowering* lowerin
     return guarded([&] {
         if (!ir) throw std::runtime_error("plan_generate: null ir");
         const ag::Plan plan = ag::parse_plan(ir);
-        ag::Lowering low = default_lowering(plan);
+        ag::Lowering low = default_lowering(plan, lowering && lowering->math >= 0 ? lowering->math : 0);
         if (lowering) {
-            if (lowering->block > 0) low.block = lowering->block;
+            if (lowering->block > 0) {
+                low.block = lowering->block;
+                low.by_size = false;
+            }
             if (lowering->ipt > 0) low.ipt = lowering->ipt;
             if (lowering->vec > 0) low.vec = lowering->vec;
             if (lowering->contract >= 0) low.contract = lowering->contract != 0;

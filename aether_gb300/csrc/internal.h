@@ -46,7 +46,9 @@ struct PlanObj {
     cudaKernel_t fv = nullptr, fs = nullptr;
     int vec = 2;
     int registers = 0;
-    int blocks_per_sm_v = 1, blocks_per_sm_s = 1;
+    // resident CTAs per SM of the two kernels at kBlocks[i] threads (at
+    // low.block, index 0, where the caller named the block)
+    int blocks_per_sm_v[4] = {1, 1, 1, 1}, blocks_per_sm_s[4] = {1, 1, 1, 1};
     int sms = 1;
     int dev = 0;
     // Default workspaces of sum plans (launches with args->workspace == NULL):
@@ -77,7 +79,9 @@ static_assert(sizeof(AgItemHost) == 648, "AgItem layout");
 struct BatchObj {
     std::vector<PlanObj*> plans;
     std::vector<int> vecs;
-    int block = 256, ipt = 1;
+    // 128 threads a CTA unless named: uneven items leave less of their last tile
+    // idle (2048 arrays, double-float: 619 us at 128, 664 at 256, 635 at 512)
+    int block = 128, ipt = 1;
     std::string name, source;
     ag::Compiled compiled;
     cudaLibrary_t library = nullptr;
@@ -101,10 +105,14 @@ inline void ag_ck(cudaError_t e, const char* what) {
     }
 }
 
-// Samples one CTA pass of a plan's kernel covers.
-inline uint64_t chunk_samples(const PlanObj& P, bool vectorized) {
-    return uint64_t(P.low.block) * uint64_t(P.low.ipt) * uint64_t(vectorized ? P.vec : 1);
-}
+// Block sizes a launch may take where the caller named none.
+constexpr int kBlocks[4] = {64, 128, 256, 512};
+
+// The shape of one launch of a plan's own kernel over n samples.
+struct PlanShape {
+    unsigned grid, block;
+};
+PlanShape plan_shape(const PlanObj& P, uint64_t n, bool vectorized);
 
 // Samples one tile of plan p of a batch covers.
 inline uint64_t batch_tile_samples(const BatchObj& B, int p) {

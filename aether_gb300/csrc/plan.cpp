@@ -1019,6 +1019,11 @@ int effective_vec(const Plan& plan, const Lowering& low) {
     return widest >= 8 ? 2 : 4;
 }
 
+int default_block(const Plan& P, int math) {
+    const bool tf = P.dst_dtype == DType::F64 && (math == 3 || (math == 0 && native_needs_tf(P)));
+    return tf && !P.wants_sum() ? 512 : 256;
+}
+
 std::string kernel_base(const Plan& plan, const std::string& text) {
     uint64_t h = 1469598103934665603ULL;
     for (unsigned char c : text) {
@@ -1127,6 +1132,7 @@ std::string generate_source(const Plan& plan_in, const Lowering& low, const std:
         if ((tfx || f64n) && (uses_trig(P) || draws_normals(P))) o << "#include \"ag_tf64_trig.cuh\"\n";
         if (low.math >= 1 && draws_normals(P)) o << "#include \"ag_emu64_bm.cuh\"\n";
         o << "#define AG_BLOCK " << low.block << "\n#define AG_IPT " << low.ipt << "\n#define AG_VEC " << vec << "\n";
+        o << "#define AG_THREADS " << (low.by_size ? "blockDim.x" : "AG_BLOCK") << "\n";
     }
     const std::string W = g.W, S = g.S;
     const int OC = P.dst_planes();   // stored planes (ff: hi then lo; acc: value then compensation)
@@ -1154,7 +1160,7 @@ std::string generate_source(const Plan& plan_in, const Lowering& low, const std:
     o << ") {\n";
     o << "    constexpr int L = AG_IPT * VEC;\n";
     o << "    ag_u64 s0[AG_IPT];\n";
-    o << "#pragma unroll\n    for (int j = 0; j < AG_IPT; ++j) s0[j] = chunk * (ag_u64)(AG_BLOCK * AG_IPT * VEC) + ((ag_u64)j * AG_BLOCK + threadIdx.x) * VEC;\n";
+    o << "#pragma unroll\n    for (int j = 0; j < AG_IPT; ++j) s0[j] = chunk * (ag_u64)(AG_THREADS * AG_IPT * VEC) + ((ag_u64)j * AG_THREADS + threadIdx.x) * VEC;\n";
     // One range check for every lane group of the thread (the last is the furthest).
     o << "    const bool full_ = s0[AG_IPT - 1] + (ag_u64)VEC <= a.n;\n";
     // Loads of every operand used in the lane context.
@@ -1371,7 +1377,7 @@ std::string generate_source(const Plan& plan_in, const Lowering& low, const std:
         const std::string name = base + (variant == 0 ? "_v" : "_s");
         const std::string V = variant == 0 ? "AG_VEC" : "1";
         k << "extern \"C\" __global__ void " << lb << " " << name << "(const AgArgs a) {\n";
-        k << "    const ag_u64 per = (ag_u64)AG_BLOCK * AG_IPT * " << V << ";\n";
+        k << "    const ag_u64 per = (ag_u64)AG_THREADS * AG_IPT * " << V << ";\n";
         k << "    const ag_u64 nchunks = (a.n + per - 1) / per;\n";
         if (sum) k << "    double h = 0.0, c = 0.0;\n";   // the thread's pair over all its chunks
         k << "    for (ag_u64 ch = blockIdx.x; ch < nchunks; ch += gridDim.x) {\n";
@@ -1415,7 +1421,7 @@ std::string generate_batch_source(const std::vector<const Plan*>& plans, const s
     if (tf || ntf) o << "#include \"ag_tf64.cuh\"\n";
     if (tft) o << "#include \"ag_tf64_trig.cuh\"\n";
     if (bm) o << "#include \"ag_emu64_bm.cuh\"\n";
-    o << "#define AG_BLOCK " << block << "\n#define AG_IPT " << ipt << "\n";
+    o << "#define AG_BLOCK " << block << "\n#define AG_IPT " << ipt << "\n#define AG_THREADS AG_BLOCK\n";
     std::vector<int> vecs;
     for (size_t p = 0; p < plans.size(); ++p) {
         if (plans[p]->wants_sum()) throw std::runtime_error("aether-ir: sum plans cannot join a batch");

@@ -52,7 +52,8 @@ struct Plan {
 
 // Lowering options (part of the cache key).
 struct Lowering {
-    int block = 256;          // threads per CTA
+    int block = 256;          // threads per CTA (at most, where by_size)
+    bool by_size = false;     // the caller left the block to the engine: each launch takes its own
     int ipt = 1;              // lane groups per thread per chunk
     int vec = 0;              // samples per lane group (0 = 16 bytes of the widest storage type)
     bool contract = true;     // allow FMA contraction of arithmetic nodes
@@ -86,5 +87,8 @@ std::string kernel_base(const Plan& plan, const std::string& text);
 
 // Chunk = samples one CTA covers per pass = block * ipt * vec.
 int effective_vec(const Plan& plan, const Lowering& low);
+
+// Threads per CTA of a plan whose caller names none.
+int default_block(const Plan& plan, int math);
 
 }  // namespace ag

@@ -387,13 +387,10 @@ struct Server {
         AetherLaunch a = launch_of(r, ops);
         AgArgsHost k;
         const bool vect = make_args(P, &a, k) && P->vec > 1;
-        const uint64_t per = chunk_samples(*P, vect);
-        const int bps = vect ? P->blocks_per_sm_v : P->blocks_per_sm_s;
-        const uint64_t cap = uint64_t(std::max(bps, 1)) * uint64_t(P->sms);
-        const unsigned grid = unsigned(std::max<uint64_t>(1, std::min((r.n + per - 1) / per, cap)));
+        const PlanShape g = plan_shape(*P, r.n, vect);
         void* params[] = {&k};
-        ag_ck(cudaLaunchKernel(reinterpret_cast<const void*>(vect ? P->fv : P->fs), dim3(grid),
-                               dim3(unsigned(P->low.block)), params, 0, stream),
+        ag_ck(cudaLaunchKernel(reinterpret_cast<const void*>(vect ? P->fv : P->fs), dim3(g.grid),
+                               dim3(g.block), params, 0, stream),
               "cudaLaunchKernel(plain)");
     }
 

@@ -467,7 +467,7 @@ __device__ __forceinline__ void sum_finish(const AgArgs& a, double h, double c) 
     __syncthreads();
     if (threadIdx.x == 0) {
         double H = sh_h[0], C = sh_c[0];
-        for (int w = 1; w < BLOCK / 32; ++w) pair_combine(H, C, sh_h[w], sh_c[w], H, C);
+        for (int w = 1; w < (int)(blockDim.x >> 5); ++w) pair_combine(H, C, sh_h[w], sh_c[w], H, C);
         double2* part = reinterpret_cast<double2*>(a.ws + 16);
         __stcg(part + blockIdx.x, make_double2(H, C));
         __threadfence();
@@ -479,7 +479,7 @@ __device__ __forceinline__ void sum_finish(const AgArgs& a, double h, double c) 
         __threadfence();
         const double2* part = reinterpret_cast<const double2*>(a.ws + 16);
         double H = 0.0, C = 0.0;
-        for (unsigned k = threadIdx.x; k < gridDim.x; k += BLOCK) {
+        for (unsigned k = threadIdx.x; k < gridDim.x; k += blockDim.x) {
             const double2 q = __ldcg(part + k);
             pair_combine(H, C, q.x, q.y, H, C);
         }
@@ -492,7 +492,7 @@ __device__ __forceinline__ void sum_finish(const AgArgs& a, double h, double c) 
         __syncthreads();
         if (threadIdx.x == 0) {
             double RH = sh_h[0], RC = sh_c[0];
-            for (int w = 1; w < BLOCK / 32; ++w) pair_combine(RH, RC, sh_h[w], sh_c[w], RH, RC);
+            for (int w = 1; w < (int)(blockDim.x >> 5); ++w) pair_combine(RH, RC, sh_h[w], sh_c[w], RH, RC);
             a.red[0] = RH;
             a.red[1] = RC;
             *reinterpret_cast<volatile unsigned*>(a.ws) = 0u;
