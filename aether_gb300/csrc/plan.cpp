@@ -1156,7 +1156,7 @@ std::string generate_source(const Plan& plan_in, const Lowering& low, const std:
 
     // The chunk body: one pass of a CTA over block*ipt*VEC consecutive samples.
     o << "template <int VEC>\n__device__ __forceinline__ void ag_chunk" << suffix << "(const AgArgs& a, ag_u64 chunk";
-    if (sum) o << (prec ? ", ag::e64::df& acc" : ", double& acc_h, double& acc_c");
+    if (sum) o << (prec ? ", ag::e64::df& acc" : ", ag::sum_acc& acc");
     o << ") {\n";
     o << "    constexpr int L = AG_IPT * VEC;\n";
     o << "    ag_u64 s0[AG_IPT];\n";
@@ -1320,9 +1320,9 @@ std::string generate_source(const Plan& plan_in, const Lowering& low, const std:
         o << "          } }\n";
     }
     if (sum) {
-        o << "        if (s0[l / VEC] + (ag_u64)(l % VEC) < a.n) ";
-        if (prec) o << "acc = ag::e64::add(acc, fv0);\n";   // per-thread float-float sum
-        else o << "ag::neumaier_add(acc_h, acc_c, (double)fv0);\n";
+        const char* in = "s0[l / VEC] + (ag_u64)(l % VEC) < a.n";
+        if (prec) o << "        if (" << in << ") acc = ag::e64::add(acc, fv0);\n";   // per-thread float-float sum
+        else o << "        acc.add(" << in << " ? (double)fv0 : 0.0);\n";
     }
     o << (G.pm ? "    }\n    }\n" : "    }\n");
     };
@@ -1379,7 +1379,8 @@ std::string generate_source(const Plan& plan_in, const Lowering& low, const std:
         k << "extern \"C\" __global__ void " << lb << " " << name << "(const AgArgs a) {\n";
         k << "    const ag_u64 per = (ag_u64)AG_THREADS * AG_IPT * " << V << ";\n";
         k << "    const ag_u64 nchunks = (a.n + per - 1) / per;\n";
-        if (sum) k << "    double h = 0.0, c = 0.0;\n";   // the thread's pair over all its chunks
+        // the thread's sum over all its chunks
+        if (sum) k << (prec ? "    double h = 0.0, c = 0.0;\n" : "    ag::sum_acc acc;\n    unsigned it = 0u;\n");
         k << "    for (ag_u64 ch = blockIdx.x; ch < nchunks; ch += gridDim.x) {\n";
         if (sum && prec) {
             // float-float within a chunk, an FP64 pair across chunks
@@ -1387,11 +1388,13 @@ std::string generate_source(const Plan& plan_in, const Lowering& low, const std:
             k << "        ag_chunk<" << V << ">(a, ch, acc);\n";
             k << "        ag::pair_combine(h, c, ag::e64::f2d(acc.hi), ag::e64::f2d(acc.lo), h, c);\n";
         } else if (sum) {
-            k << "        ag_chunk<" << V << ">(a, ch, h, c);\n";
+            k << "        ag_chunk<" << V << ">(a, ch, acc);\n";
+            k << "        if ((++it & 1023u) == 0u) acc.flush();\n";   // at most 32 terms a chunk
         } else {
             k << "        ag_chunk<" << V << ">(a, ch);\n";
         }
-        k << (sum ? "    }\n    ag::sum_finish<AG_BLOCK>(a, h, c);\n}\n" : "    }\n}\n");
+        k << (!sum ? "    }\n}\n" : prec ? "    }\n    ag::sum_finish<AG_BLOCK>(a, h, c);\n}\n"
+                                          : "    }\n    acc.flush();\n    ag::sum_finish<AG_BLOCK>(a, acc.h, acc.c);\n}\n");
     }
     return k.str();
 }

@@ -407,6 +407,78 @@ __device__ __forceinline__ void butterfly32(T& h, T& c) {
     }
 }
 
+// The pair (h, c) plus a 128-bit integer in units of 2^(base - 1075): its four
+// words as exact doubles of one sign, the largest first. Out of line: it runs
+// a few times per thread.
+__device__ __noinline__ double2 sum_flush(double h, double c, ag_u32 w0, ag_u32 w1, ag_u32 w2, ag_u32 w3, int base) {
+    const bool neg = (int)w3 < 0;
+    if (neg) {
+        const ag_u64 lo = ~((ag_u64)w1 << 32 | w0) + 1ull, hi = ~((ag_u64)w3 << 32 | w2) + (lo == 0ull ? 1ull : 0ull);
+        w0 = (ag_u32)lo, w1 = (ag_u32)(lo >> 32), w2 = (ag_u32)hi, w3 = (ag_u32)(hi >> 32);
+    }
+    const ag_u32 w[4] = {w3, w2, w1, w0};
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        if (!w[k]) continue;
+        const double unit = __hiloint2double((int)((ag_u32)(base - 52 + 32 * (3 - k)) << 20), 0);
+        const double t = __dmul_rn((double)w[k], unit);
+        neumaier_add(h, c, neg ? -t : t);
+    }
+    return make_double2(h, c);
+}
+// One thread's sum of doubles: a 128-bit integer in units of 2^(base - 1075)
+// and a compensated FP64 pair. A term whose exponent lies in the integer's
+// window [base, base + 58] is shifted into place and added there, exactly, in
+// some 20 integer operations where the pair takes four on the FP64 pipe (67
+// clocks a warp, more than the terms of a dot product cost): the sum of 2^25
+// three-component f64 dot products went from 459 to 263 us. A term above the
+// window moves it (the warp's largest exponent sets it, so that all lanes move
+// at once); one below it, a subnormal, an infinity or a NaN joins the pair.
+// Any number of magnitudes is summed no less exactly than by the pair alone.
+struct sum_acc {
+    double h, c;
+    ag_u32 w0, w1, w2, w3;
+    int base;
+
+    __device__ __forceinline__ sum_acc() : h(0.0), c(0.0), w0(0u), w1(0u), w2(0u), w3(0u), base(-(1 << 20)) {}
+    __device__ __forceinline__ void flush() {
+        const double2 r = sum_flush(h, c, w0, w1, w2, w3, base);
+        h = r.x;
+        c = r.y;
+        w0 = w1 = w2 = w3 = 0u;
+    }
+    // All lanes of the warp call it together. At most 2^15 terms between flushes.
+    __device__ __forceinline__ void add(double x) {
+        const ag_u32 xh = (ag_u32)__double2hiint(x), xl = (ag_u32)__double2loint(x);
+        const int e = (int)((xh >> 20) & 0x7ffu);
+        int sh = e - base;
+        if (__any_sync(0xffffffffu, sh > 58 && e < 2047)) {
+            flush();
+            // the largest finite exponent sits 4 below the window's top
+            const int top = __reduce_max_sync(0xffffffffu, e < 2047 ? e : 0);
+            base = top - 54 > 53 ? top - 54 : 53;
+            sh = e - base;
+        }
+        if ((unsigned)sh <= 58u && e != 0 && e < 2047) {
+            const ag_u32 mh = (xh & 0xfffffu) | 0x100000u;
+            const ag_u32 f0 = xl << (sh & 31), f1 = __funnelshift_l(xl, mh, (unsigned)sh), f2 = __funnelshift_l(mh, 0u, (unsigned)sh);
+            const bool up = sh >= 32;
+            const ag_u32 neg = (ag_u32)((int)xh >> 31);
+            const ag_u32 a0 = (up ? 0u : f0) ^ neg, a1 = (up ? f0 : f1) ^ neg, a2 = (up ? f1 : f2) ^ neg, a3 = (up ? f2 : 0u) ^ neg;
+            ag_u32 one;   // the two's complement's +1 as the first carry
+            asm("add.cc.u32 %4, %9, 1;\n\t"
+                "addc.cc.u32 %0, %0, %5;\n\t"
+                "addc.cc.u32 %1, %1, %6;\n\t"
+                "addc.cc.u32 %2, %2, %7;\n\t"
+                "addc.u32 %3, %3, %8;"
+                : "+r"(w0), "+r"(w1), "+r"(w2), "+r"(w3), "=r"(one)
+                : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(neg));
+        } else if (xh << 1 | xl) {
+            neumaier_add(h, c, x);
+        }
+    }
+};
+
 }  // namespace ag
 
 namespace ag {
