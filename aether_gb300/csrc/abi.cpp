@@ -131,6 +131,14 @@ ag::Lowering default_lowering(const ag::Plan& p, int math) {
     return l;
 }
 
+// A caller that names a block, or another part of the kernel's shape that sets
+// its registers, gets one fixed block (256 threads if none is named).
+void set_block(ag::Lowering& l, const AetherLowering& given) {
+    if (given.block <= 0 && given.ipt <= 0 && given.vec <= 0 && given.min_blocks <= 0) return;
+    l.block = given.block > 0 ? given.block : 256;
+    l.by_size = false;
+}
+
 uint64_t ws_needed(const PlanObj& P, uint64_t n) {
     if (!P.plan.wants_sum()) return 0;
     // one partial for each of the scalar kernel's chunks at low.block threads, the
@@ -322,10 +330,7 @@ AG_EXPORT int aether_plan_create(const char* ir, const AetherLowering* lowering,
         P->plan = ag::parse_plan(ir);
         P->low = default_lowering(P->plan, lowering && lowering->math >= 0 ? lowering->math : 0);
         if (lowering) {
-            if (lowering->block > 0) {
-                P->low.block = lowering->block;
-                P->low.by_size = false;
-            }
+            set_block(P->low, *lowering);
             if (lowering->ipt > 0) P->low.ipt = lowering->ipt;
             if (lowering->vec > 0) P->low.vec = lowering->vec;
             if (lowering->contract >= 0) P->low.contract = lowering->contract != 0;
@@ -358,7 +363,7 @@ AG_EXPORT int aether_plan_create(const char* ir, const AetherLowering* lowering,
         cudaFuncAttributes fa{};
         ck(cudaFuncGetAttributes(&fa, reinterpret_cast<const void*>(P->fv)), "cudaFuncGetAttributes");
         P->registers = fa.numRegs;
-        for (int i = 0; i < (P->low.by_size ? 4 : 1); ++i) {
+        for (int i = 0; i < (P->low.by_size ? kNumBlocks : 1); ++i) {
             const int block = P->low.by_size ? std::min(kBlocks[i], P->low.block) : P->low.block;
             ck(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&P->blocks_per_sm_v[i],
                                                              reinterpret_cast<const void*>(P->fv), block, 0), "occupancy");
@@ -386,7 +391,7 @@ AG_EXPORT int aether_plan_info(void* plan, AetherPlanInfo* info) {
         info->vec = P->vec;
         info->registers = P->registers;
         info->blocks_per_sm = P->blocks_per_sm_v[0];
-        for (int i = 0; P->low.by_size && i < 4; ++i)
+        for (int i = 0; P->low.by_size && i < kNumBlocks; ++i)
             if (kBlocks[i] <= P->low.block) info->blocks_per_sm = P->blocks_per_sm_v[i];
         info->compile_ms = P->compiled.compile_ms;
     });
@@ -414,20 +419,27 @@ AG_EXPORT int aether_plan_source(void* plan, char* buf, size_t cap, size_t* len)
 }
 
 // Where the caller named no block: the largest that still gives every SM
-// enough CTAs, so that a small launch spreads over the chip. Triple-float
-// kernels (blocks of up to 512) want one per SM: their CTAs run in step through
-// long straight-line code (plain fused expression, 2^24 x 3: 885 us at 512
-// threads, 952 at 256, 975 at 64; 4099 samples: 10.7, 7.3 and 6.5 us). The
-// others want 16 (inverses: 4.9 us at 256 and 3.5 at 64 threads for 4099
-// samples, 41.8 and 39.1 at 128 for 2^20; sums of 65536 terms 14.4 and 11.4 us;
-// from 2^24 samples on all sizes are within 1 %).
+// enough CTAs. One CTA of 768 threads per SM runs its warps in step through
+// long straight-line code and through neighbouring lines (2^24 x 3 samples at
+// 768 and 256 threads: large streaming expression 359 and 390 us in
+// double-float, 798 and 874 at FP64 grade; plain fused expression 490 and 521 in
+// double-float; N(0, 1) draws 142 and 153), once 24 of them
+// follow one another, which keeps the last wave's idle SMs below 4 %. Smaller
+// launches spread over the chip: triple-float kernels want one CTA of 512 per
+// SM (plain fused expression, 4099 samples: 10.7, 7.3 and 6.5 us at 512, 256
+// and 64 threads), the others 16 of 256 (3x3 inverses, 4099 samples: 4.9 us at
+// 256 and 3.5 at 64; sums of 65536 terms 14.4 and 11.4 us).
 PlanShape plan_shape(const PlanObj& P, uint64_t n, bool vectorized) {
     const uint64_t lanes = uint64_t(P.low.ipt) * uint64_t(vectorized ? P.vec : 1);
     int block = P.low.block, i = 0;
     if (P.low.by_size) {
-        const uint64_t want = (block > 256 ? 1 : 16) * uint64_t(P.sms);
-        for (i = 3; i > 0; --i)
-            if (kBlocks[i] <= P.low.block && (n + kBlocks[i] * lanes - 1) / (kBlocks[i] * lanes) >= want) break;
+        const bool tf = ag::triple_float(P.plan, P.low.math) && !P.plan.wants_sum();
+        for (i = kNumBlocks - 1; i > 0; --i) {
+            if (kBlocks[i] > P.low.block || (kBlocks[i] == 512 && !tf)) continue;
+            const int bps = vectorized ? P.blocks_per_sm_v[i] : P.blocks_per_sm_s[i];
+            const uint64_t want = uint64_t(kBlocks[i] == 768 ? 24 * std::max(bps, 1) : tf ? 1 : 16) * uint64_t(P.sms);
+            if ((n + kBlocks[i] * lanes - 1) / (kBlocks[i] * lanes) >= want) break;
+        }
         block = kBlocks[i];
     }
     uint64_t chunks = (n + uint64_t(block) * lanes - 1) / (uint64_t(block) * lanes);
@@ -787,10 +799,7 @@ AG_EXPORT int aether_plan_generate(const char* ir, const AetherLowering* lowerin
         const ag::Plan plan = ag::parse_plan(ir);
         ag::Lowering low = default_lowering(plan, lowering && lowering->math >= 0 ? lowering->math : 0);
         if (lowering) {
-            if (lowering->block > 0) {
-                low.block = lowering->block;
-                low.by_size = false;
-            }
+            set_block(low, *lowering);
             if (lowering->ipt > 0) low.ipt = lowering->ipt;
             if (lowering->vec > 0) low.vec = lowering->vec;
             if (lowering->contract >= 0) low.contract = lowering->contract != 0;

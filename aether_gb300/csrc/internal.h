@@ -48,7 +48,7 @@ struct PlanObj {
     int registers = 0;
     // resident CTAs per SM of the two kernels at kBlocks[i] threads (at
     // low.block, index 0, where the caller named the block)
-    int blocks_per_sm_v[4] = {1, 1, 1, 1}, blocks_per_sm_s[4] = {1, 1, 1, 1};
+    int blocks_per_sm_v[5] = {1, 1, 1, 1, 1}, blocks_per_sm_s[5] = {1, 1, 1, 1, 1};
     int sms = 1;
     int dev = 0;
     // Default workspaces of sum plans (launches with args->workspace == NULL):
@@ -106,7 +106,8 @@ inline void ag_ck(cudaError_t e, const char* what) {
 }
 
 // Block sizes a launch may take where the caller named none.
-constexpr int kBlocks[4] = {64, 128, 256, 512};
+constexpr int kNumBlocks = 5;
+constexpr int kBlocks[kNumBlocks] = {64, 128, 256, 512, 768};
 
 // The shape of one launch of a plan's own kernel over n samples.
 struct PlanShape {

@@ -1019,11 +1019,6 @@ int effective_vec(const Plan& plan, const Lowering& low) {
     return widest >= 8 ? 2 : 4;
 }
 
-int default_block(const Plan& P, int math) {
-    const bool tf = P.dst_dtype == DType::F64 && (math == 3 || (math == 0 && native_needs_tf(P)));
-    return tf && !P.wants_sum() ? 512 : 256;
-}
-
 std::string kernel_base(const Plan& plan, const std::string& text) {
     uint64_t h = 1469598103934665603ULL;
     for (unsigned char c : text) {
@@ -1071,6 +1066,25 @@ bool draws_normals(const Plan& P) {
     for (const Node& n : P.nodes)
         if (n.op == "normal" || n.op == "lognormal") return true;
     return false;
+}
+
+bool triple_float(const Plan& P, int math) {
+    return P.dst_dtype == DType::F64 && (math == 3 || (math == 0 && native_needs_tf(P)));
+}
+
+int default_block(const Plan& P, int math) {
+    // Sums end in a tree over their CTAs; light fills and native trees without
+    // ag::n64 are bound by HBM and Philox (uniform draws, 3 components, 10^7
+    // samples: 61 us compiled for 256 threads, 68 for 768) and may hold many
+    // components of f32 samples (3x3 inverses, 8 10^6: 99 us against 315 when
+    // squeezed into 80 registers).
+    const bool tf = triple_float(P, math);
+    if (P.wants_sum() || (math == 0 && !tf) || (P.has_random && !heavy(P))) return 256;
+    // 768 threads leave a thread 80 registers: too few for a matrix of
+    // triple-floats (3x3 inverses, 2^24: 894 us at 512 threads, 1065 at 768) and
+    // for native trees on middling sizes (plain fused expression, 2^20 x 3: 62
+    // us with 112 registers, 66 with 80)
+    return tf && (math == 0 || P.dst_comps >= 9) ? 512 : 768;
 }
 
 std::string generate_source(const Plan& plan_in, const Lowering& low, const std::string& base,

@@ -88,7 +88,11 @@ std::string kernel_base(const Plan& plan, const std::string& text);
 // Chunk = samples one CTA covers per pass = block * ipt * vec.
 int effective_vec(const Plan& plan, const Lowering& low);
 
-// Threads per CTA of a plan whose caller names none.
+// Most threads per CTA of a plan whose caller names none.
 int default_block(const Plan& plan, int math);
+
+// Whether the plan's values are triple-floats (FP64-grade plans, and native ones
+// that call ag::n64).
+bool triple_float(const Plan& plan, int math);
 
 }  // namespace ag
