@@ -341,6 +341,7 @@ AG_EXPORT int aether_plan_create(const char* ir, const AetherLowering* lowering,
             throw std::runtime_error("plan_create: block must be a multiple of 32 in [32, 1024]");
         if (P->low.ipt < 1 || P->low.ipt > 8) throw std::runtime_error("plan_create: ipt must be in [1, 8]");
         P->vec = ag::effective_vec(P->plan, P->low);
+        P->tf = ag::triple_float(P->plan, P->low.math) && !P->plan.wants_sum();
         if (P->vec != 1 && P->vec != 2 && P->vec != 4) throw std::runtime_error("plan_create: vec must be 1, 2 or 4");
         if (P->low.math == 1 && P->plan.dst_dtype != ag::DType::F64)
             throw std::runtime_error("plan_create: emulated FP64 (math = 1) applies to f64 plans");
@@ -433,11 +434,10 @@ PlanShape plan_shape(const PlanObj& P, uint64_t n, bool vectorized) {
     const uint64_t lanes = uint64_t(P.low.ipt) * uint64_t(vectorized ? P.vec : 1);
     int block = P.low.block, i = 0;
     if (P.low.by_size) {
-        const bool tf = ag::triple_float(P.plan, P.low.math) && !P.plan.wants_sum();
         for (i = kNumBlocks - 1; i > 0; --i) {
-            if (kBlocks[i] > P.low.block || (kBlocks[i] == 512 && !tf)) continue;
+            if (kBlocks[i] > P.low.block || (kBlocks[i] == 512 && !P.tf)) continue;
             const int bps = vectorized ? P.blocks_per_sm_v[i] : P.blocks_per_sm_s[i];
-            const uint64_t want = uint64_t(kBlocks[i] == 768 ? 24 * std::max(bps, 1) : tf ? 1 : 16) * uint64_t(P.sms);
+            const uint64_t want = uint64_t(kBlocks[i] == 768 ? 24 * std::max(bps, 1) : P.tf ? 1 : 16) * uint64_t(P.sms);
             if ((n + kBlocks[i] * lanes - 1) / (kBlocks[i] * lanes) >= want) break;
         }
         block = kBlocks[i];

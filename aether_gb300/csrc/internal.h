@@ -45,6 +45,7 @@ struct PlanObj {
     cudaLibrary_t library = nullptr;
     cudaKernel_t fv = nullptr, fs = nullptr;
     int vec = 2;
+    bool tf = false;   // ag::triple_float, sums aside
     int registers = 0;
     // resident CTAs per SM of the two kernels at kBlocks[i] threads (at
     // low.block, index 0, where the caller named the block)

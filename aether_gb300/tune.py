@@ -25,7 +25,7 @@ DEFAULT_CANDIDATES = [
     for v in (0, 1)
     for m in (0, 2, 3, 4)
     if not (b == 512 and m == 4) and not (b < 512 and m == 2)   # 512 x 2 CTAs caps a thread at 64 registers
-]
+] + [dict(block=b, ipt=1, vec=0, min_blocks=0) for b in (768, 1024)]   # one CTA per SM, its warps in step
 
 
 def cache_path():
