@@ -273,25 +273,14 @@ class Launch:
 
     def __init__(self, plan, ctx, n, dst_ptr, dst_pitch, sample_offset=0, reduce_ptr=None, workspace=None):
         self.plan = plan
-        self._ops = (_abi.AetherOperand * max(1, len(ctx.operands)))()
-        for i, (ptr, pitch, _dt, _c, _owner) in enumerate(ctx.operands):
-            self._ops[i].ptr = ptr
-            self._ops[i].pitch = pitch
-        self._owners = [o[4] for o in ctx.operands]
-        self._sc = (ctypes.c_double * max(1, len(ctx.scalars)))(*ctx.scalars)
-        self._keys = (ctypes.c_uint64 * max(1, len(ctx.keys)))(*ctx.keys)
-        a = _abi.AetherLaunch()
-        a.n = n
-        a.sample_offset = sample_offset
-        a.dst = dst_ptr or 0
-        a.dst_pitch = dst_pitch
-        a.operands = self._ops
-        a.n_operands = len(ctx.operands)
-        a.scalars = self._sc
-        a.n_scalars = len(ctx.scalars)
-        a.keys = self._keys
-        a.n_keys = len(ctx.keys)
-        a.reduce_out = reduce_ptr or 0
+        operands, scalars, keys = ctx.operands, ctx.scalars, ctx.keys
+        self._ops = (_abi.AetherOperand * max(1, len(operands)))(*[o[:2] for o in operands])
+        self._owners = [o[4] for o in operands]
+        self._sc = (ctypes.c_double * max(1, len(scalars)))(*scalars)
+        self._keys = (ctypes.c_uint64 * max(1, len(keys)))(*keys)
+        # in the order of the struct's fields
+        a = _abi.AetherLaunch(n, sample_offset, 0, dst_ptr or 0, dst_pitch, self._ops, len(operands), self._sc,
+                              len(scalars), self._keys, len(keys), reduce_ptr or 0)
         if workspace is not None:
             a.workspace = workspace.data_ptr()
             a.workspace_bytes = workspace.numel() * workspace.element_size()

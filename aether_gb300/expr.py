@@ -36,10 +36,11 @@ class IrContext:
 
     def operand(self, leaf):
         k = (leaf.ptr, leaf.pitch, leaf.dtype, leaf.comps)
-        if k not in self._op_index:
-            self._op_index[k] = len(self.operands)
-            self.operands.append((leaf.ptr, leaf.pitch, leaf.dtype, leaf.comps, leaf.owner))
-        return self._op_index[k]
+        i = self._op_index.get(k)
+        if i is None:
+            i = self._op_index[k] = len(self.operands)
+            self.operands.append(k + (leaf.owner,))
+        return i
 
     def scalar(self, v):
         self.scalars.append(float(v))
@@ -227,12 +228,23 @@ class Node(Expr):
         self.ints = tuple(ints)
         self.tail_text = tail_text
 
+    # Writing a small statement's text is most of what assign() does on the
+    # host: 9 us of the plain fused expression's 19 before the launch itself,
+    # 19 of 29 when the leaves' own texts were put together on each call.
     def ir(self, ctx):
-        parts = [k.ir(ctx) for k in self.kids]
-        parts += [str(i) for i in self.ints]
+        kids = self.kids
+        n = len(kids)
+        if n == 2:
+            t = "(" + self.op + " " + kids[0].ir(ctx) + " " + kids[1].ir(ctx)
+        elif n == 1:
+            t = "(" + self.op + " " + kids[0].ir(ctx)
+        else:
+            t = "(" + self.op + " " + " ".join([k.ir(ctx) for k in kids])
+        for i in self.ints:
+            t += " " + str(i)
         if self.tail_text:
-            parts.append(self.tail_text)
-        return "(" + self.op + " " + " ".join(parts) + ")"
+            t += " " + self.tail_text
+        return t + ")"
 
 
 class Operand(Expr):
@@ -246,9 +258,10 @@ class Operand(Expr):
         self.comps = _prod(self.shape)
         self.owner = owner
         self.is_bool = dtype == "u8"
+        self._type_text = " " + dtype + " " + _shape_text(self.shape) + ")"
 
     def ir(self, ctx):
-        return "(in %d %s %s)" % (ctx.operand(self), self.dtype, _shape_text(self.shape))
+        return "(in " + str(ctx.operand(self)) + self._type_text
 
 
 class Scalar(Expr):
