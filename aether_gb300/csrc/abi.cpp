@@ -442,14 +442,15 @@ PlanShape plan_shape(const PlanObj& P, uint64_t n, bool vectorized) {
         }
         block = kBlocks[i];
     }
-    uint64_t chunks = (n + uint64_t(block) * lanes - 1) / (uint64_t(block) * lanes);
+    const uint64_t chunks = (n + uint64_t(block) * lanes - 1) / (uint64_t(block) * lanes);
+    uint64_t ctas = chunks;
     if (P.plan.wants_sum()) {   // no more partials than the workspace of n samples holds
         const uint64_t per = uint64_t(P.low.block) * uint64_t(P.low.ipt);
-        chunks = std::min(chunks, (n + per - 1) / per);
+        ctas = std::min(ctas, (n + per - 1) / per);
     }
     const int bps = vectorized ? P.blocks_per_sm_v[i] : P.blocks_per_sm_s[i];
     const uint64_t cap = uint64_t(std::max(bps, 1)) * uint64_t(P.sms);
-    return PlanShape{unsigned(std::max<uint64_t>(1, std::min(chunks, cap))), unsigned(block)};
+    return PlanShape{unsigned(std::max<uint64_t>(1, std::min(ctas, cap))), unsigned(block), uint32_t(chunks)};
 }
 
 // Internal (not exported): lets other translation units of the library report
@@ -509,6 +510,7 @@ namespace {
 
 void launch_plan_kernel(const PlanObj& P, AgArgsHost& k, uint64_t n, bool vect, cudaStream_t s) {
     const PlanShape g = plan_shape(P, n, vect);
+    k.chunks = g.chunks;
     void* params[] = {&k};
     ck(cudaLaunchKernel(reinterpret_cast<const void*>(vect ? P.fv : P.fs), dim3(g.grid), dim3(g.block), params, 0, s),
        "cudaLaunchKernel");

@@ -21,7 +21,7 @@
 // receives it by value.
 struct AgArgsHost {
     uint64_t n;
-    uint32_t offset, flags;
+    uint32_t offset, chunks;
     char* dst;
     uint64_t dst_pitch;
     const char* ops[16];
@@ -113,6 +113,7 @@ constexpr int kBlocks[kNumBlocks] = {64, 128, 256, 512, 768};
 // The shape of one launch of a plan's own kernel over n samples.
 struct PlanShape {
     unsigned grid, block;
+    uint32_t chunks;   // for AgArgs
 };
 PlanShape plan_shape(const PlanObj& P, uint64_t n, bool vectorized);
 

@@ -1391,11 +1391,9 @@ std::string generate_source(const Plan& plan_in, const Lowering& low, const std:
         const std::string name = base + (variant == 0 ? "_v" : "_s");
         const std::string V = variant == 0 ? "AG_VEC" : "1";
         k << "extern \"C\" __global__ void " << lb << " " << name << "(const AgArgs a) {\n";
-        k << "    const ag_u64 per = (ag_u64)AG_THREADS * AG_IPT * " << V << ";\n";
-        k << "    const ag_u64 nchunks = (a.n + per - 1) / per;\n";
         // the thread's sum over all its chunks
         if (sum) k << (prec ? "    double h = 0.0, c = 0.0;\n" : "    ag::sum_acc acc;\n    unsigned it = 0u;\n");
-        k << "    for (ag_u64 ch = blockIdx.x; ch < nchunks; ch += gridDim.x) {\n";
+        k << "    for (ag_u64 ch = blockIdx.x; ch < a.chunks; ch += gridDim.x) {\n";
         if (sum && prec) {
             // float-float within a chunk, an FP64 pair across chunks
             k << "        ag::e64::df acc = ag::e64::mk(0.0f, 0.0f);\n";

@@ -391,6 +391,7 @@ struct Server {
         AgArgsHost k;
         const bool vect = make_args(P, &a, k) && P->vec > 1;
         const PlanShape g = plan_shape(*P, r.n, vect);
+        k.chunks = g.chunks;
         void* params[] = {&k};
         ag_ck(cudaLaunchKernel(reinterpret_cast<const void*>(vect ? P->fv : P->fs), dim3(g.grid),
                                dim3(g.block), params, 0, stream),

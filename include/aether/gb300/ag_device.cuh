@@ -22,7 +22,7 @@ typedef long long ag_i64;
 struct AgArgs {
     ag_u64 n;                     // samples
     ag_u32 offset;                // global sample id of sample 0 (Philox position)
-    ag_u32 flags;
+    ag_u32 chunks;                // chunks of the launch (n < 2^32): a plan's kernel need not divide by its block
     char* dst;                    // plane 0 of the destination
     ag_u64 dst_pitch;             // elements between planes
     const char* ops[AG_MAX_OPS];  // plane 0 of each operand
