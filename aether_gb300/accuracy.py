@@ -19,11 +19,13 @@ abs+rel of cuRAND's (tests/random/golden_random.h:437-441), which is about
 9007 x 2^-53.
 """
 
-# Native FP64 lowering (math 0): CUDA's FP64 functions. Arithmetic and
+# Native FP64 lowering (math 0): FP64 arithmetic; square roots, reciprocal
+# roots and quotients correctly rounded and exp, log, log1p, sin and cos within
+# 0.6 ulp of exact from triple-float, CUDA's functions for the rest. Arithmetic and
 # geometry are bit-exact with contraction off; a transcendental expression
 # stays within this many ulp of its largest term (spacing of the term scale).
 NATIVE_EXPR_ULPS = 4
-# Native Box-Muller normals (CUDA's FP64 log, sqrt and sin), abs+rel in 2^-53.
+# Native Box-Muller normals (log, sqrt and sin each rounded from triple-float), abs+rel in 2^-53.
 NATIVE_NORMAL_BOUND_2M53 = 8
 
 # Emulated FP64 lowering (math 1): double-float arithmetic on the FP32/INT

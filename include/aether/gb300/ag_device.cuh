@@ -525,7 +525,8 @@ __device__ __forceinline__ int next_item(const Item* __restrict__ items, int n_i
 // (about 45 FP64 operations a thread) runs once per CTA. It ran once per chunk
 // before, which cost three times the sum itself: 2^26 8-component float dot
 // products with their global sum went from 2.67 to 0.70 ms (98 % of measured
-// HBM), the sum of 2^25 3-component f64 ones from 2.68 to 0.46 ms (FP64 pipe).
+// HBM), the sum of 2^25 3-component f64 ones from 2.68 to 0.46 ms (0.26 with
+// sum_acc's window).
 template <int BLOCK>
 __device__ __forceinline__ void sum_finish(const AgArgs& a, double h, double c) {
     __shared__ double sh_h[BLOCK / 32], sh_c[BLOCK / 32];

@@ -541,7 +541,7 @@ namespace y64 = t64;   // the spelling of a plan's two-sample code
 // function out of line. Measured: a + b c + sin(a) exp(-c c) over 2^20
 // three-component samples, 232 us with CUDA's functions, 65 us with these; a
 // fill of 3 uniform components and one N(0, 1) draw for 10^7 samples, 1555 and
-// 294 us.
+// 267 us.
 // ---------------------------------------------------------------------------
 namespace n64 {
 using t64::tf;

@@ -118,7 +118,9 @@ typedef struct AetherLowering {
     int ipt;          /* lane groups per thread per chunk */
     int vec;          /* samples per lane group (vector width) */
     int contract;     /* 1: FMA contraction allowed, 0: every add/mul rounds (-fmad=false), -1: default (1) */
-    int math;         /* 0: FP64 on the FP64 pipe; 1: FP64 emulated on the FP32/INT pipes (double-float);
+    int math;         /* 0: native FP64 (division, roots, exp, logarithms, sine, cosine and normal draws
+                         rounded from triple-float, the rest on the FP64 pipe);
+                         1: FP64 emulated on the FP32/INT pipes (double-float);
                          2: the precision form -- f32 or float-float storage evaluated in double-float
                          arithmetic, exact products of f32 operands, FP64 only in the final stage of sums;
                          3: FP64-grade on the FP32/INT pipes (triple-float, f64 plans): doubles split exactly
