@@ -605,14 +605,18 @@ __device__ __forceinline__ auto join(tfT<F> v) {
     typename lanes<F>::whole i;
     return join(v, g, i);
 }
-// The same, clearing `ok` within 2^-9 of an ulp of a rounding boundary (the
-// triple-float sqrt, recip and quotient are good to 2^-12 of one).
+// The same, clearing `ok` within 2^-12 of an ulp of a rounding boundary (the
+// triple-float sqrt and recip are good to 2^-15 of one, the quotient to 2^-14).
+// One lane in 2048 then takes the function out of line. 2^-9 sent one in 256,
+// some lane of every eighth warp, to 20 FP64 operations and more: the large
+// streaming expression over 2^24 x 3 samples took 1180 us so, 945 now, 3x3
+// inverses of 2^22 samples 282 and 237.
 template <class F>
 __device__ __forceinline__ auto join_exact(tfT<F> v, typename lanes<F>::flag& ok) {
     F g;
     typename lanes<F>::whole i;
     const auto r = join(v, g, i);
-    e64::within(fsub(g, e64::to_f(i)), -0.498046875f, 0.498046875f, ok);
+    e64::within(fsub(g, e64::to_f(i)), -0.499755859375f, 0.499755859375f, ok);
     return r;
 }
 
