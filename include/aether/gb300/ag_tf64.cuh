@@ -536,7 +536,8 @@ namespace y64 = t64;   // the spelling of a plan's two-sample code
 // 60 operations on it) bound every plan that calls one; these use none of it.
 // sqrt, rsqrt and div are correctly rounded: a value closer to a rounding
 // boundary than the evaluation's own error is handed to the FP64 pipe. log,
-// log1p, exp, sin and cos are within 0.51 ulp, under CUDA's 1 to 2. Arguments
+// log1p, exp, sin and cos are within 0.52 ulp (sin and cos 0.59 beside
+// multiples of pi/2), under CUDA's 1 to 2. Arguments
 // outside the triple-float range, zeros, infinities and NaN take CUDA's
 // function out of line. Measured: a + b c + sin(a) exp(-c c) over 2^20
 // three-component samples, 232 us with CUDA's functions, 65 us with these; a
