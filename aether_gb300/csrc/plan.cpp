@@ -523,6 +523,36 @@ struct Gen {
         }
         return sum_only_memo[size_t(id)] != 0;
     }
+    // Triple-floats: whether node `id`'s lower floats may overlap its upper ones
+    // by more than a few bits. A sum that cancels leaves them so, and products,
+    // quotients and roots of such a value do too; functions that reduce their
+    // argument do not.
+    std::vector<signed char> overlap_memo;
+    bool overlaps(int id) {
+        static const std::set<std::string> none = {"in", "sc", "lit", "lognormal", "exponential", "bernoulli",
+                                                   "pow", "pows", "atan2", "hypot"};
+        static const std::set<std::string> as_kids = {
+            "bcast", "at0", "comp", "seg", "row", "col", "transpose", "block", "reshape", "stack", "neg", "abs", "qconj",
+            "pureq", "select", "min", "max", "mins", "maxs", "clamp", "sq", "mul", "scale", "outer", "div", "sqrt",
+            "rsqrt", "sqnorm", "norm", "rnorm", "unit", "maxnorm"};
+        if (overlap_memo.empty()) overlap_memo.assign(P.nodes.size(), -1);
+        signed char& m = overlap_memo[size_t(id)];
+        if (m >= 0) return m != 0;
+        const Node& n = P.nodes[size_t(id)];
+        const std::string& op = n.op;
+        bool r = true;
+        if (as_kids.count(op) || (op == "add" && nonneg(n.kids[0]) && nonneg(n.kids[1]))) {
+            r = false;
+            for (size_t j = op == "select" ? 1 : 0; j < n.kids.size(); ++j) r = r || overlaps(n.kids[j]);
+        } else if (op == "normal") {   // N(0, 1) is the draw itself
+            const Node &mean = P.nodes[size_t(n.kids[0])], &dev = P.nodes[size_t(n.kids[1])];
+            r = !(mean.op == "lit" && mean.lit == 0.0 && dev.op == "lit" && dev.lit == 1.0);
+        } else if (none.count(op) || unary_ops().count(op)) {
+            r = false;
+        }
+        m = r ? 1 : 0;
+        return r;
+    }
     std::string sqr(bool u, const std::string& x) { return (u ? NS + "sqr_u(" : NS + "sqr(") + x + ")"; }
 
     std::string add(const std::string& a, const std::string& b) const {
@@ -1226,13 +1256,18 @@ std::string generate_source(const Plan& plan_in, const Lowering& low, const std:
     // over 2^23 x 3 152 and 125 us, 3x3 inverses 421 and 273 us. A
     // triple-float's five operations are never hidden (stream 959 and 861 us
     // for 2^24 x 3, inverses 753 and 457 us).
-    const std::string to_dbl = tfx || (!prec && !heavy(P)) ? "out_double(" : "to_double(";
+    const std::string to_dbl = !prec && !heavy(P) ? "out_double(" : "to_double(";
     // The output range test is left out when the magnitude bounds of the root
     // keep every value of a lane that passed its other checks inside [2^-88,
     // 2^126), and a NaN (the root of a negative number) stays one: a float
     // pair's, or one reassembled on the FP64 pipe. In integers it would not.
     auto out_safe = [&](Gen& G) {
+        if (tfx) return G.lo_of(P.root) >= -80 && G.hi_of(P.root) <= 125;   // right for every value, NaN among them
         return emu && to_dbl == "to_double(" && G.lo_of(P.root) >= -88 && G.hi_of(P.root) <= 125;
+    };
+    // A triple-float's reassembly, with its range test.
+    auto tf_out = [&](Gen& G, const std::string& v) {
+        return G.NS + "out_double(" + (G.overlaps(P.root) ? G.NS + "renorm(" + v + ")" : v) + (out_safe(G) ? ")" : ", ok_)");
     };
     // One lane loop: the values of each sample, then what is done with them.
     std::vector<std::string> root;
@@ -1249,16 +1284,16 @@ std::string generate_source(const Plan& plan_in, const Lowering& low, const std:
         // from here on one sample at a time
         const bool dbl = emu && !prec;   // the values leave as doubles
         const std::string fn = G.dfm ? "ag::e64::ln" : "ag::ln", T1 = dbl ? "double" : G.W1;
-        if (dbl && !out_safe(G))
+        if (dbl && !tfx && !out_safe(G))
             for (int c = 0; c < P.dst_comps; ++c) o << "        " << G.NS << "out_double_ok(" << root[size_t(c)] << ", ok_);\n";
-        if (emu) o << "        const ag::e64::b2 okp_ = ok_;\n";
         for (int c = 0; c < P.dst_comps; ++c) {
             const std::string n = std::to_string(c), r = root[size_t(c)];
-            if (dbl) o << "        const ag::e64::d2 rd" << n << " = " << G.NS << to_dbl << r << ");\n";
+            if (dbl) o << "        const ag::e64::d2 rd" << n << " = " << (tfx ? tf_out(G, r) : G.NS + to_dbl + r + ")") << ";\n";
             o << "        const " << T1 << " ra" << n << " = " << (dbl ? "rd" + n + ".a" : fn + "0(" + r + ")") << ", rb" << n << " = "
               << (dbl ? "rd" + n + ".b" : fn + "1(" + r + ")") << ";\n";
             root[size_t(c)] = "r" + n;
         }
+        if (emu) o << "        const ag::e64::b2 okp_ = ok_;\n";
         o << "#pragma unroll\n        for (int k_ = 0; k_ < 2; ++k_) {\n        const int l = lp + k_;\n";
         if (emu) o << "        bool ok_ = k_ ? okp_.b : okp_.a;\n";
         for (int c = 0; c < P.dst_comps; ++c)
@@ -1273,6 +1308,8 @@ std::string generate_source(const Plan& plan_in, const Lowering& low, const std:
             if (!out_safe(G)) o << "        ok_ = ok_ && ag::e64::out_ok(fv" << c << ");\n";
         } else if (emu && G.pm) {
             o << "        double fv" << c << " = " << root[size_t(c)] << ";\n";
+        } else if (tfx) {
+            o << "        double fv" << c << " = " << tf_out(G, root[size_t(c)]) << ";\n";
         } else if (emu) {
             o << "        double fv" << c << " = " << G.NS << to_dbl << root[size_t(c)] << ");\n";
             if (!out_safe(G)) o << "        " << G.NS << "out_double_ok(" << root[size_t(c)] << ", ok_);\n";

@@ -451,15 +451,19 @@ __device__ __forceinline__ void within(f2 x, float lo, float hi, b2& ok) {
 // A float and what is left of a value, joined to a double with integer
 // operations: the double of x, plus the rest in units of its last place.
 // ---------------------------------------------------------------------------
-// 2^(52 - e) for |x| in [2^e, 2^(e+1)), with x's sign, from x's exponent field;
-// twice that where x is a power of two and the rest (of w's sign) leads below
-// it, where the double's unit halves. Needs |x| in [2^-75, 2^127).
+// 2^(52 - DOWN - e) for |x| in [2^e, 2^(e+1)), with x's sign, from x's exponent
+// field; twice that where x is a power of two and the rest (of w's sign) leads
+// below it, where the double's unit halves. Needs |x| in [2^(-75-DOWN), 2^127).
+template <unsigned DOWN = 0>
 __device__ __forceinline__ float join_scale(float x, float w) {
     const unsigned xb = (unsigned)__float_as_int(x), wb = (unsigned)__float_as_int(w);
     const bool down = (xb & 0x7fffffu) == 0u && (wb & 0x7fffffffu) != 0u && ((wb ^ xb) >> 31) != 0u;
-    return __int_as_float((int)(((down ? 307u : 306u) << 23) - (xb & 0x7f800000u) + (xb & 0x80000000u)));
+    return __int_as_float((int)(((down ? 307u - DOWN : 306u - DOWN) << 23) - (xb & 0x7f800000u) + (xb & 0x80000000u)));
 }
-__device__ __forceinline__ f2 join_scale(f2 x, f2 w) { return pk(join_scale(ln0(x), ln0(w)), join_scale(ln1(x), ln1(w))); }
+template <unsigned DOWN = 0>
+__device__ __forceinline__ f2 join_scale(f2 x, f2 w) {
+    return pk(join_scale<DOWN>(ln0(x), ln0(w)), join_scale<DOWN>(ln1(x), ln1(w)));
+}
 // The double of x, `off` units further from zero.
 __device__ __forceinline__ double join_bits(float x, int off) {
     const unsigned xb = (unsigned)__float_as_int(x);

@@ -131,8 +131,8 @@ __device__ __forceinline__ tfT<F> add_lead(tfT<F> a, tfT<F> b) {
     const dfT<F> w = fast_two_sum(s.hi, u.hi);
     return mk3(w.hi, w.lo, z);
 }
-// The reassembly into a double rounds x + y + z once whatever their overlap,
-// so the root of a plan has no cheaper form here.
+// A plan's root has no cheaper form here: its reassembly in integers wants the
+// first two floats normalised.
 template <class F>
 __device__ __forceinline__ tfT<F> add_fast_u(tfT<F> a, tfT<F> b) { return add_fast(a, b); }
 
@@ -181,8 +181,8 @@ __device__ __forceinline__ tfT<F> sqr_df(dfT<F> a) {
     const dfT<F> w = fast_two_sum(p.hi, u.hi);
     return mk3(w.hi, w.lo, z);
 }
-// Products read only by sums: the reassembly and every sum above take any
-// overlap, so the same value serves.
+// Products read only by sums: every sum above takes any overlap, so the same
+// value serves.
 template <class F>
 __device__ __forceinline__ tfT<F> sqr_u(tfT<F> a) { return sqr(a); }
 
@@ -696,15 +696,87 @@ __device__ __forceinline__ d2 div(d2 x, d2 y) {
 }  // namespace n64
 
 namespace t64 {
-// A plan's output: x + y + z rounded once, without the FP64 pipe (five
-// operations of it in to_double).
-template <class F>
-__device__ __forceinline__ auto out_double(tfT<F> v) {
-    return n64::join(v);
+// Whether x + y + z can be put together in integers, given Y and Z, its lower
+// parts in twice the unit of the double's last place: |x| in [2^-74, 2^127),
+// |Y| <= 2^28 (the next float's distance: the sum stays in x's binade), and
+// |Z| <= 2^8, so that a float holds what is rounded to 2^-15 of a unit. False
+// for a NaN.
+__device__ __forceinline__ bool join_fits(float x, float Y, float Z) {
+    const unsigned e = ((unsigned)__float_as_int(x) >> 23) & 0xffu;
+    return e - 53u <= 200u && fabsf(Y) <= 268435456.0f && fabsf(Z) <= 256.0f;
+}
+__device__ __forceinline__ b2 join_fits(f2 x, f2 Y, f2 Z) {
+    return b2{join_fits(ln0(x), ln0(Y), ln0(Z)), join_fits(ln1(x), ln1(Y), ln1(Z))};
+}
+#if defined(__CUDACC__) || defined(__CUDACC_RTC__)
+// Out of line: predicated, its five FP64 operations would issue for every warp
+// with a zero in it.
+__device__ __noinline__ double slow_sum(float x, float y, float z) { return to_double(mk3(x, y, z)); }
+#else
+__device__ __forceinline__ double slow_sum(float x, float y, float z) { return to_double(mk3(x, y, z)); }
+#endif
+// Zeros, which sparse results have many of, need no sum.
+__device__ __forceinline__ void or_sum(bool fits, tf v, double& r) {
+    if (!fits) {
+        const unsigned xb = (unsigned)__float_as_int(v.x), yb = (unsigned)__float_as_int(v.y), zb = (unsigned)__float_as_int(v.z);
+        r = __hiloint2double((int)(xb & yb & zb), 0);
+        if (((xb | yb | zb) & 0x7fffffffu) != 0u) r = slow_sum(v.x, v.y, v.z);
+    }
+}
+__device__ __forceinline__ void or_sum(bool fits, tf v, double& r, bool& ok) {
+    if (!fits) {
+        ok = ok && out_ok(v);
+        if (ok) r = slow_sum(v.x, v.y, v.z);
+    }
+}
+__device__ __forceinline__ void or_sum(b2 fits, tf2 v, e64::d2& r) {
+    if (!(fits.a && fits.b)) {
+        or_sum(fits.a, ln0(v), r.a);
+        or_sum(fits.b, ln1(v), r.b);
+    }
+}
+__device__ __forceinline__ void or_sum(b2 fits, tf2 v, e64::d2& r, b2& ok) {
+    if (!(fits.a && fits.b)) {
+        or_sum(fits.a, ln0(v), r.a, ok.a);
+        or_sum(fits.b, ln1(v), r.b, ok.b);
+    }
+}
+// A plan's output: x + y + z rounded once to nearest even, without the FP64
+// pipe (five operations of it in to_double) where the parts overlap no more
+// than an operation on normalised operands leaves them; to_double otherwise.
+// Right for every value; a sum that may cancel is handed over renormalised so
+// that it takes the integers (renorm is 12 FP32 operations). Y is rounded to an
+// even number of units and what is left by an addition to 1.5 2^22, whose last
+// place is half of Y's unit, so that a tie goes to the even double.
+__device__ __forceinline__ int half_units(float g) { return __float_as_int(__fadd_rn(g, 6291456.0f)) - 0x4AC00000; }
+__device__ __forceinline__ i2 half_units(f2 g) {
+    const f2 t = fadd(g, bc<f2>(6291456.0f));
+    return i2{__float_as_int(ln0(t)) - 0x4AC00000, __float_as_int(ln1(t)) - 0x4AC00000};
 }
 template <class F>
-__device__ __forceinline__ void out_double_ok(tfT<F> v, typename lanes<F>::flag& ok) {
-    e64::out_range(v.x, ok);
+__device__ __forceinline__ auto out_join(tfT<F> v, typename lanes<F>::flag& fits) {
+    const F S = e64::join_scale<1>(v.x, fadd(v.y, v.z));
+    const F Y = fmul(v.y, S), Z = fmul(v.z, S);   // exact scalings
+    const typename lanes<F>::whole h = e64::to_int(Y);
+    const F g = fadd(fsub(Y, e64::to_f(h)), Z);
+    fits = join_fits(v.x, Y, Z);
+    return e64::join_bits(v.x, e64::plus(e64::plus(h, h), half_units(g)));
+}
+template <class F>
+__device__ __forceinline__ auto out_double(tfT<F> v) {
+    typename lanes<F>::flag fits;
+    auto r = out_join(v, fits);
+    or_sum(fits, v, r);
+    return r;
+}
+// The same for a value that may have left the range: `ok` is cleared where
+// out_ok is false.
+template <class F>
+__device__ __forceinline__ auto out_double(tfT<F> v, typename lanes<F>::flag& ok) {
+    typename lanes<F>::flag fits;
+    auto r = out_join(v, fits);
+    or_sum(fits, v, r, ok);
+    return r;
 }
 }  // namespace t64
 #endif
