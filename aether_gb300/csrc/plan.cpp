@@ -1256,18 +1256,23 @@ std::string generate_source(const Plan& plan_in, const Lowering& low, const std:
     // over 2^23 x 3 152 and 125 us, 3x3 inverses 421 and 273 us. A
     // triple-float's five operations are never hidden (stream 959 and 861 us
     // for 2^24 x 3, inverses 753 and 457 us).
-    const std::string to_dbl = !prec && !heavy(P) ? "out_double(" : "to_double(";
+    const bool joins = tfx || (!prec && !heavy(P));
     // The output range test is left out when the magnitude bounds of the root
     // keep every value of a lane that passed its other checks inside [2^-88,
-    // 2^126), and a NaN (the root of a negative number) stays one: a float
-    // pair's, or one reassembled on the FP64 pipe. In integers it would not.
-    auto out_safe = [&](Gen& G) {
-        if (tfx) return G.lo_of(P.root) >= -80 && G.hi_of(P.root) <= 125;   // right for every value, NaN among them
-        return emu && to_dbl == "to_double(" && G.lo_of(P.root) >= -88 && G.hi_of(P.root) <= 125;
+    // 2^126) (2^-80 for triple-floats). Either reassembly is right for every
+    // value, a NaN (the root of a negative number) among them.
+    auto out_safe = [&](Gen& G) { return emu && G.lo_of(P.root) >= (tfx ? -80 : -88) && G.hi_of(P.root) <= 125; };
+    // The reassembly of v, and the range test before it (out_double of a
+    // triple-float holds its own).
+    auto dbl_out = [&](Gen& G, const std::string& v) -> std::string {
+        if (tfx)
+            return G.NS + "out_double(" + (G.overlaps(P.root) ? G.NS + "renorm(" + v + ")" : v) + (out_safe(G) ? ")" : ", ok_)");
+        return G.NS + (!joins ? "to_double(" : out_safe(G) ? "out_double(" : "out_join(") + v + ")";
     };
-    // A triple-float's reassembly, with its range test.
-    auto tf_out = [&](Gen& G, const std::string& v) {
-        return G.NS + "out_double(" + (G.overlaps(P.root) ? G.NS + "renorm(" + v + ")" : v) + (out_safe(G) ? ")" : ", ok_)");
+    auto dbl_test = [&](Gen& G, const std::string& v) -> std::string {
+        if (tfx || out_safe(G)) return "";
+        return joins ? "        " + G.NS + "out_double_ok(" + v + ", ok_);\n"
+                     : "        ok_ = ag::e64::both_of(ok_, " + G.NS + "out_ok(" + v + "));\n";
     };
     // One lane loop: the values of each sample, then what is done with them.
     std::vector<std::string> root;
@@ -1284,11 +1289,10 @@ std::string generate_source(const Plan& plan_in, const Lowering& low, const std:
         // from here on one sample at a time
         const bool dbl = emu && !prec;   // the values leave as doubles
         const std::string fn = G.dfm ? "ag::e64::ln" : "ag::ln", T1 = dbl ? "double" : G.W1;
-        if (dbl && !tfx && !out_safe(G))
-            for (int c = 0; c < P.dst_comps; ++c) o << "        " << G.NS << "out_double_ok(" << root[size_t(c)] << ", ok_);\n";
+        for (int c = 0; dbl && c < P.dst_comps; ++c) o << dbl_test(G, root[size_t(c)]);
         for (int c = 0; c < P.dst_comps; ++c) {
             const std::string n = std::to_string(c), r = root[size_t(c)];
-            if (dbl) o << "        const ag::e64::d2 rd" << n << " = " << (tfx ? tf_out(G, r) : G.NS + to_dbl + r + ")") << ";\n";
+            if (dbl) o << "        const ag::e64::d2 rd" << n << " = " << dbl_out(G, r) << ";\n";
             o << "        const " << T1 << " ra" << n << " = " << (dbl ? "rd" + n + ".a" : fn + "0(" + r + ")") << ", rb" << n << " = "
               << (dbl ? "rd" + n + ".b" : fn + "1(" + r + ")") << ";\n";
             root[size_t(c)] = "r" + n;
@@ -1308,11 +1312,9 @@ std::string generate_source(const Plan& plan_in, const Lowering& low, const std:
             if (!out_safe(G)) o << "        ok_ = ok_ && ag::e64::out_ok(fv" << c << ");\n";
         } else if (emu && G.pm) {
             o << "        double fv" << c << " = " << root[size_t(c)] << ";\n";
-        } else if (tfx) {
-            o << "        double fv" << c << " = " << tf_out(G, root[size_t(c)]) << ";\n";
         } else if (emu) {
-            o << "        double fv" << c << " = " << G.NS << to_dbl << root[size_t(c)] << ");\n";
-            if (!out_safe(G)) o << "        " << G.NS << "out_double_ok(" << root[size_t(c)] << ", ok_);\n";
+            o << "        double fv" << c << " = " << dbl_out(G, root[size_t(c)]) << ";\n";
+            o << dbl_test(G, root[size_t(c)]);
         } else {
             o << "        const " << G.W1 << " fv" << c << " = " << root[size_t(c)] << ";\n";
         }

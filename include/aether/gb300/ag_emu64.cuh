@@ -411,6 +411,9 @@ __device__ __forceinline__ bool out_ok(df v) {
     const unsigned e = ((unsigned)__float_as_int(v.hi) >> 23) & 0xffu;
     return e - 37u <= 216u;   // |hi| in [2^-90, 2^127)
 }
+__device__ __forceinline__ bool both_of(bool x, bool y) { return x && y; }
+__device__ __forceinline__ b2 both_of(b2 x, b2 y) { return b2{x.a && y.a, x.b && y.b}; }
+__device__ __forceinline__ b2 out_ok(df2 v) { return b2{out_ok(ln0(v)), out_ok(ln1(v))}; }
 __device__ __forceinline__ d2 to_double(df2 v) { return d2{to_double(ln0(v)), to_double(ln1(v))}; }
 // 0 < w < 2^54 as a double-float: the top 24 significant bits exactly, the
 // rest rounded once (2^-48 relative).
@@ -453,7 +456,7 @@ __device__ __forceinline__ void within(f2 x, float lo, float hi, b2& ok) {
 // ---------------------------------------------------------------------------
 // 2^(52 - DOWN - e) for |x| in [2^e, 2^(e+1)), with x's sign, from x's exponent
 // field; twice that where x is a power of two and the rest (of w's sign) leads
-// below it, where the double's unit halves. Needs |x| in [2^(-75-DOWN), 2^127).
+// below it, where the double's unit halves. Needs |x| in [2^(-74-DOWN), 2^127).
 template <unsigned DOWN = 0>
 __device__ __forceinline__ float join_scale(float x, float w) {
     const unsigned xb = (unsigned)__float_as_int(x), wb = (unsigned)__float_as_int(w);
@@ -473,26 +476,64 @@ __device__ __forceinline__ double join_bits(float x, int off) {
 __device__ __forceinline__ d2 join_bits(f2 x, i2 off) { return d2{join_bits(ln0(x), off.a), join_bits(ln1(x), off.b)}; }
 __device__ __forceinline__ int to_int(float x) { return __float2int_rn(x); }
 __device__ __forceinline__ i2 to_int(f2 x) { return i2{to_int(ln0(x)), to_int(ln1(x))}; }
+// Whether join_bits and join_scale<DOWN> hold for x: |x| in [2^(-74-DOWN), 2^127).
+template <unsigned DOWN>
+__device__ __forceinline__ bool join_head(float x) {
+    const unsigned e = ((unsigned)__float_as_int(x) >> 23) & 0xffu;
+    return e - (53u - DOWN) <= 200u + DOWN;
+}
+template <unsigned DOWN>
+__device__ __forceinline__ b2 join_head(f2 x) {
+    return b2{join_head<DOWN>(ln0(x)), join_head<DOWN>(ln1(x))};
+}
 // hi + lo rounded once, as to_double gives it, without the FP64 pipe: its two
 // conversions and one addition are 50 clocks a warp there, which alone held the
 // large streaming expression at 73 clocks an element and the batched cross
-// products, rotations and inverses at 79 % of that pipe.
+// products, rotations and inverses at 79 % of that pipe. For |hi + lo| in
+// [2^-94, 2^127): the scale alone would leave the floats below 2^-75, so 2^20 of
+// it is a factor of its own (by sample: as a pair it took the batched kernel
+// from 94 to 98 registers, five CTAs to four, 622 to 673 us).
+__device__ __forceinline__ int units_20(float x) { return to_int(__fmul_rn(x, 1048576.0f)); }
+__device__ __forceinline__ i2 units_20(f2 x) { return i2{units_20(ln0(x)), units_20(ln1(x))}; }
+template <class F>
+__device__ __forceinline__ auto out_join(dfT<F> v) {
+    const dfT<F> n = fast_two_sum(v.hi, v.lo);   // |lo| <= half an ulp of hi: no carry past its binade
+    return join_bits(n.hi, units_20(fmul(n.lo, join_scale<20>(n.hi, n.lo))));
+}
+#if defined(__CUDACC__) || defined(__CUDACC_RTC__)
+// Out of line: predicated, its FP64 operations would issue for every warp with
+// a zero in it.
+__device__ __noinline__ double slow_sum(float hi, float lo) { return to_double(mk(hi, lo)); }
+#else
+__device__ __forceinline__ double slow_sum(float hi, float lo) { return to_double(mk(hi, lo)); }
+#endif
+// Zeros, which sparse results have many of, need no sum.
+__device__ __forceinline__ void or_sum(bool fits, df v, double& r) {
+    if (!fits) {
+        const unsigned hb = (unsigned)__float_as_int(v.hi), lb = (unsigned)__float_as_int(v.lo);
+        r = __hiloint2double((int)(hb & lb), 0);
+        if (((hb | lb) & 0x7fffffffu) != 0u) r = slow_sum(v.hi, v.lo);
+    }
+}
+__device__ __forceinline__ void or_sum(b2 fits, df2 v, d2& r) {
+    if (!(fits.a && fits.b)) {
+        or_sum(fits.a, ln0(v), r.a);
+        or_sum(fits.b, ln1(v), r.b);
+    }
+}
+// A plan's output, right for every value: heads out of range, zeros and NaN
+// take the FP64 sum.
 template <class F>
 __device__ __forceinline__ auto out_double(dfT<F> v) {
-    const dfT<F> n = fast_two_sum(v.hi, v.lo);   // |lo| <= half an ulp of hi: no carry past its binade
-    return join_bits(n.hi, to_int(fmul(n.lo, join_scale(n.hi, n.lo))));
+    auto r = out_join(v);
+    or_sum(join_head<20>(fadd(v.hi, v.lo)), v, r);
+    return r;
 }
-__device__ __forceinline__ void out_range(float x, bool& ok) {   // |x| in [2^-75, 2^127)
-    const unsigned e = ((unsigned)__float_as_int(x) >> 23) & 0xffu;
-    ok = ok && e - 52u <= 201u;
-}
-__device__ __forceinline__ void out_range(f2 x, b2& ok) {
-    out_range(ln0(x), ok.a);
-    out_range(ln1(x), ok.b);
-}
+// For values that may have left the range, out_join after this test: the lane
+// runs natively where it fails.
 template <class F>
 __device__ __forceinline__ void out_double_ok(dfT<F> v, typename lanes<F>::flag& ok) {
-    out_range(fadd(v.hi, v.lo), ok);
+    ok = both_of(ok, out_ok(mk(fadd(v.hi, v.lo), v.lo)));
 }
 #endif
 

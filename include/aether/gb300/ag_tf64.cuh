@@ -697,13 +697,12 @@ __device__ __forceinline__ d2 div(d2 x, d2 y) {
 
 namespace t64 {
 // Whether x + y + z can be put together in integers, given Y and Z, its lower
-// parts in twice the unit of the double's last place: |x| in [2^-74, 2^127),
+// parts in twice the unit of the double's last place: |x| in [2^-75, 2^127),
 // |Y| <= 2^28 (the next float's distance: the sum stays in x's binade), and
 // |Z| <= 2^8, so that a float holds what is rounded to 2^-15 of a unit. False
 // for a NaN.
 __device__ __forceinline__ bool join_fits(float x, float Y, float Z) {
-    const unsigned e = ((unsigned)__float_as_int(x) >> 23) & 0xffu;
-    return e - 53u <= 200u && fabsf(Y) <= 268435456.0f && fabsf(Z) <= 256.0f;
+    return e64::join_head<1>(x) && fabsf(Y) <= 268435456.0f && fabsf(Z) <= 256.0f;
 }
 __device__ __forceinline__ b2 join_fits(f2 x, f2 Y, f2 Z) {
     return b2{join_fits(ln0(x), ln0(Y), ln0(Z)), join_fits(ln1(x), ln1(Y), ln1(Z))};
