@@ -1242,8 +1242,9 @@ std::string generate_source(const Plan& plan_in, const Lowering& low, const std:
     }
     if (P.has_random) o << "    const ag_u32 g0 = a.offset;\n";
     if (emu) o << "    bool ok0_ = true;\n";
-    // Plain assignments recompute their out-of-range lanes after the stores,
-    // keeping the native call out of the lane loop.
+    // Plain assignments recompute their out-of-range lanes after the stores of
+    // the others, keeping the native call out of the lane loop. It reads its
+    // sample's operands again, and the destination may be one of them.
     const bool defer = emu && P.op == "set" && store;
     if (defer) o << "    unsigned bad_ = 0u;\n";
     o << g.pro.str();
@@ -1390,14 +1391,18 @@ std::string generate_source(const Plan& plan_in, const Lowering& low, const std:
     if (pairs) o << "    }\n";
     if (store) {
         o << "    " << S << "* __restrict__ po = (" << S << "*)a.dst;\n";
-        o << "    if (full_) {\n#pragma unroll\n    for (int c = 0; c < " << OC << "; ++c)\n#pragma unroll\n        for (int j = 0; j < AG_IPT; ++j) ag::vec_io<VEC, " << S
-          << ">::store_full(po + c * a.dst_pitch, s0[j], &out[c][j * VEC]);\n    } else {\n";
-        o << "#pragma unroll\n    for (int c = 0; c < " << OC << "; ++c)\n#pragma unroll\n        for (int j = 0; j < AG_IPT; ++j) ag::vec_io<VEC, " << S
-          << ">::store(po + c * a.dst_pitch, s0[j], a.n, &out[c][j * VEC]);\n    }\n";
+        const std::string rows = "#pragma unroll\n    for (int c = 0; c < " + std::to_string(OC) + "; ++c)\n#pragma unroll\n";
+        const std::string io = "        for (int j = 0; j < AG_IPT; ++j) ag::vec_io<VEC, " + S + ">::";
+        if (defer) o << "    if (bad_ == 0u) {\n";
+        o << "    if (full_) {\n" << rows << io << "store_full(po + c * a.dst_pitch, s0[j], &out[c][j * VEC]);\n    } else {\n"
+          << rows << io << "store(po + c * a.dst_pitch, s0[j], a.n, &out[c][j * VEC]);\n    }\n";
+        if (defer)   // the thread's good samples; the others' operands stay as they are until they are read again
+            o << "    } else {\n" << rows << "        for (int l = 0; l < L; ++l)\n"
+              << "            if (!((bad_ >> l) & 1u) && s0[l / VEC] + (ag_u64)(l % VEC) < a.n) (po + c * a.dst_pitch)[s0[l / VEC] + (ag_u64)(l % VEC)] = out[c][l];\n";
     }
     if (defer) {
-        // the native recomputation overwrites the lanes the fast path could not serve
-        o << "    if (bad_) {\n        " << S << "* __restrict__ pf_ = (" << S << "*)a.dst;\n";
+        // the native recomputation of the lanes the fast path could not serve
+        o << "        " << S << "* __restrict__ pf_ = (" << S << "*)a.dst;\n";
         o << "        for (int l = 0; l < L; ++l) {\n";
         o << "            const ag_u64 sl_ = s0[l / VEC] + (ag_u64)(l % VEC);\n";
         o << "            if (((bad_ >> l) & 1u) && sl_ < a.n) {\n";
