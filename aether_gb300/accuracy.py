@@ -21,7 +21,8 @@ abs+rel of cuRAND's (tests/random/golden_random.h:437-441), which is about
 
 # Native FP64 lowering (math 0): FP64 arithmetic; square roots, reciprocal
 # roots and quotients correctly rounded and exp, log, log1p, sin and cos within
-# 0.6 ulp of exact from triple-float, CUDA's functions for the rest. Arithmetic and
+# 0.52 ulp of exact (sin and cos 0.76 beside multiples of pi/2) from
+# triple-float, CUDA's functions for the rest. Arithmetic and
 # geometry are bit-exact with contraction off; a transcendental expression
 # stays within this many ulp of its largest term (spacing of the term scale).
 NATIVE_EXPR_ULPS = 4
