@@ -353,17 +353,29 @@ AG_EXPORT int aether_plan_create(const char* ir, const AetherLowering* lowering,
             throw std::runtime_error("plan_create: FP64-grade triple-float (math = 3) applies to f64 plans");
         if (P->low.math < 0 || P->low.math > 3) throw std::runtime_error("plan_create: math must be 0, 1, 2 or 3");
         P->name = ag::kernel_base(P->plan, ir) + lowering_tag(P->plan, P->low);
-        P->source = ag::generate_source(P->plan, P->low, P->name);
         ck(cudaFree(nullptr), "CUDA context");   // make the primary context current
         cudaGetDevice(&P->dev);
-        P->compiled = ag::compile_cached(P->source, "plan");
-        ck(cudaLibraryLoadData(&P->library, P->compiled.cubin.data(), nullptr, nullptr, 0, nullptr, nullptr, 0),
-           "cudaLibraryLoadData");
-        ck(cudaLibraryGetKernel(&P->fv, P->library, (P->name + "_v").c_str()), "cudaLibraryGetKernel");
-        ck(cudaLibraryGetKernel(&P->fs, P->library, (P->name + "_s").c_str()), "cudaLibraryGetKernel");
-        cudaFuncAttributes fa{};
-        ck(cudaFuncGetAttributes(&fa, reinterpret_cast<const void*>(P->fv)), "cudaFuncGetAttributes");
-        P->registers = fa.numRegs;
+        double compile_ms = 0.0;
+        for (;;) {
+            P->source = ag::generate_source(P->plan, P->low, P->name);
+            P->compiled = ag::compile_cached(P->source, "plan");
+            compile_ms += P->compiled.compile_ms;
+            ck(cudaLibraryLoadData(&P->library, P->compiled.cubin.data(), nullptr, nullptr, 0, nullptr, nullptr, 0),
+               "cudaLibraryLoadData");
+            ck(cudaLibraryGetKernel(&P->fv, P->library, (P->name + "_v").c_str()), "cudaLibraryGetKernel");
+            ck(cudaLibraryGetKernel(&P->fs, P->library, (P->name + "_s").c_str()), "cudaLibraryGetKernel");
+            cudaFuncAttributes fa{}, fs{};
+            ck(cudaFuncGetAttributes(&fa, reinterpret_cast<const void*>(P->fv)), "cudaFuncGetAttributes");
+            ck(cudaFuncGetAttributes(&fs, reinterpret_cast<const void*>(P->fs)), "cudaFuncGetAttributes");
+            P->registers = fa.numRegs;
+            if (!P->low.by_size) break;
+            const int block = ag::narrower_block(P->plan, P->low.block, std::max(fa.localSizeBytes, fs.localSizeBytes));
+            if (block == P->low.block) break;
+            P->low.block = block;
+            ck(cudaLibraryUnload(P->library), "cudaLibraryUnload");
+            P->library = nullptr;
+        }
+        P->compiled.compile_ms = compile_ms;
         for (int i = 0; i < (P->low.by_size ? kNumBlocks : 1); ++i) {
             const int block = P->low.by_size ? std::min(kBlocks[i], P->low.block) : P->low.block;
             ck(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&P->blocks_per_sm_v[i],

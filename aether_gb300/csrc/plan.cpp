@@ -1117,6 +1117,13 @@ int default_block(const Plan& P, int math) {
     return tf && (math == 0 || P.dst_comps >= 9) ? 512 : 768;
 }
 
+int narrower_block(const Plan& P, int block, size_t local_bytes) {
+    // 8 bytes a component for the native lane's values and some 100 for the
+    // functions' own frames; what is above them are spills.
+    if (block <= 256 || local_bytes <= 8u * unsigned(P.dst_comps) + 128u) return block;
+    return heavy(P) ? 512 : 256;
+}
+
 std::string generate_source(const Plan& plan_in, const Lowering& low, const std::string& base,
                             const std::string& suffix, bool chunk_only) {
     // Re-derive the sample contexts (at0 subtrees) from the node graph: every

@@ -91,6 +91,21 @@ int effective_vec(const Plan& plan, const Lowering& low);
 // Most threads per CTA of a plan whose caller names none.
 int default_block(const Plan& plan, int math);
 
+// The threads per CTA to compile for after `block` left a thread `local_bytes`
+// of local memory; `block` itself if that is no more than the plan needs.
+// A wide tree does not fit the registers of 768 threads (80 each): compiled for
+// 768 and for the block taken here, us for 2^24 elements in all,
+//                                  math 1      math 2      math 3
+//   plain fused expr., 6 comps   205 -> 206  190 -> 157  435 -> 368
+//                      9         533 -> 238  416 -> 210  (512 at once)
+//   large streaming,   6         170 -> 151  136 -> 115  407 -> 299
+//                      9         484 -> 191  375 -> 134  (512)
+//   a b - c d,         6         135 -> 106   75 ->  53  154 -> 124
+//                      9         202 -> 109  239 ->  54  (512) 170 -> 160
+// Trees with a function keep 512 (128 registers), where 256 take 5 to 20 %
+// longer on such sizes; the others are bound by HBM at 256.
+int narrower_block(const Plan& plan, int block, size_t local_bytes);
+
 // Whether the plan's values are triple-floats (FP64-grade plans, and native ones
 // that call ag::n64).
 bool triple_float(const Plan& plan, int math);
