@@ -384,6 +384,7 @@ AG_EXPORT int aether_plan_create(const char* ir, const AetherLowering* lowering,
                                                              reinterpret_cast<const void*>(P->fs), block, 0), "occupancy");
         }
         cudaDeviceGetAttribute(&P->sms, cudaDevAttrMultiProcessorCount, P->dev);
+        if (P->low.by_size) P->one_sample = ag::one_sample_limit(P->plan, P->low.math) * uint64_t(P->sms);
         *out = P.release();
     });
 }
@@ -577,7 +578,7 @@ AG_EXPORT int aether_plan_launch(void* plan, const AetherLaunch* a, void* stream
         AgArgsHost k;
         const bool aligned = make_args(P, a, k);
         cudaStream_t s = static_cast<cudaStream_t>(stream);
-        const bool vect = aligned && P->vec > 1;
+        const bool vect = vector_kernel(*P, a->n, aligned);
         if (pl.wants_sum()) {
             if (!a->reduce_out) throw std::runtime_error("plan_launch: sum plan without reduce_out");
             k.red = a->reduce_out;

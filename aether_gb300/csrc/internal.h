@@ -46,6 +46,7 @@ struct PlanObj {
     cudaKernel_t fv = nullptr, fs = nullptr;
     int vec = 2;
     bool tf = false;   // ag::triple_float, sums aside
+    uint64_t one_sample = 0;   // launches of up to so many samples run fs
     int registers = 0;
     // resident CTAs per SM of the two kernels at kBlocks[i] threads (at
     // low.block, index 0, where the caller named the block)
@@ -116,6 +117,11 @@ struct PlanShape {
     uint32_t chunks;   // for AgArgs
 };
 PlanShape plan_shape(const PlanObj& P, uint64_t n, bool vectorized);
+
+// Whether a launch of n samples takes the vector kernel, its planes aligned or not.
+inline bool vector_kernel(const PlanObj& P, uint64_t n, bool aligned) {
+    return aligned && P.vec > 1 && n > P.one_sample;
+}
 
 // Samples one tile of plan p of a batch covers.
 inline uint64_t batch_tile_samples(const BatchObj& B, int p) {

@@ -1117,6 +1117,16 @@ int default_block(const Plan& P, int math) {
     return tf && (math == 0 || P.dst_comps >= 9) ? 512 : 768;
 }
 
+bool two_samples(const Plan& P, int math) {
+    const bool f64 = P.dst_dtype == DType::F64;
+    return ((math == 1 && f64) || (math == 2 && !f64) || triple_float(P, math)) && pairable(P);
+}
+
+uint64_t one_sample_limit(const Plan& P, int math) {
+    if (P.wants_sum() || !two_samples(P, math)) return 0;
+    return heavy(P) && !triple_float(P, math) ? 2048 : 512;
+}
+
 int narrower_block(const Plan& P, int block, size_t local_bytes) {
     // 8 bytes a component for the native lane's values and some 100 for the
     // functions' own frames; what is above them are spills.
@@ -1160,7 +1170,7 @@ std::string generate_source(const Plan& plan_in, const Lowering& low, const std:
     // The same tree two samples at a time, for the lane counts it divides: the
     // FP32-pipe arithmetic of the emulated lowerings and of ag::n64 takes one
     // issue slot and half the code for both (ag_emu64.cuh).
-    const bool pairs = (emu || (P.dst_dtype == DType::F64 && native_needs_tf(P))) && pairable(P);
+    const bool pairs = two_samples(P, low.math);
     Gen gp(P, low, ctx, emu, "q", false, tfx, pairs);
     gp.root_to_double = g.root_to_double;
     if (pairs) gp.emit(P.root);

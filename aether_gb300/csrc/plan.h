@@ -106,6 +106,16 @@ int default_block(const Plan& plan, int math);
 // longer on such sizes; the others are bound by HBM at 256.
 int narrower_block(const Plan& plan, int block, size_t local_bytes);
 
+// Launches of up to this many samples per SM run the one-sample kernel even
+// where the planes are aligned (0: none do). A plan with two samples in a
+// register pair is one dependent chain twice as long as it has to be while the
+// chip has warps to spare. 16384 elements, pairs and single samples, and before
+// there were pairs (us): N(0, 1) draws in double-float 2.9, 2.4 and 2.7; a b - c d
+// over f32 at math 2 3.0, 2.1 and 2.7; large streaming expression over eight
+// f32 at math 2 9.9, 4.8 and 9.7. They meet at 500 to 700 samples per SM in
+// triple-float and without a function, near 2000 in double-float with one.
+uint64_t one_sample_limit(const Plan& plan, int math);
+
 // Whether the plan's values are triple-floats (FP64-grade plans, and native ones
 // that call ag::n64).
 bool triple_float(const Plan& plan, int math);

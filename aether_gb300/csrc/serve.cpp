@@ -389,7 +389,7 @@ struct Server {
         PlanObj* P = plans[size_t(r.plan)];
         AetherLaunch a = launch_of(r, ops);
         AgArgsHost k;
-        const bool vect = make_args(P, &a, k) && P->vec > 1;
+        const bool vect = vector_kernel(*P, r.n, make_args(P, &a, k));
         const PlanShape g = plan_shape(*P, r.n, vect);
         k.chunks = g.chunks;
         void* params[] = {&k};
