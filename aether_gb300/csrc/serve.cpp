@@ -16,6 +16,8 @@
 // only after its last checkpoint has fired, so its staging and its work list
 // are no longer read by the device when they are written again.
 
+#include <cuda.h>
+
 #include <algorithm>
 #include <chrono>
 #include <condition_variable>
@@ -369,7 +371,6 @@ struct Server {
         S.cp_end.push_back(end);
     }
 
-    // The host output copies of requests [b, e) of a slot.
     // Outputs of requests [b, e) to the host, on the slot's stream, but for those
     // that their kernels write there themselves.
     void copy_outputs(Slot& S, size_t b, size_t e) {
@@ -703,20 +704,34 @@ constexpr uint64_t kDirectOutput = 8ull << 20;
 
 uint64_t planes_of(ag::DType d, int comps) { return uint64_t(comps) * (d == ag::DType::FF ? 2u : 1u); }
 
-// Whether [p, p + bytes) is pinned host memory the device reads at the same
-// address (16-byte aligned at the start): checked at both ends.
+// Whether [p, p + bytes) lies in one allocation or registration of pinned host
+// memory that the device reads and writes at the same address, 16-byte aligned
+// at the start. (Two registrations may have unmapped pages between them, so it
+// takes the whole range's word, not that of its ends.)
 bool mapped_host(const void* p, uint64_t bytes) {
     if (!bytes || (reinterpret_cast<uintptr_t>(p) & 15u)) return false;
-    const char* ends[2] = {static_cast<const char*>(p), static_cast<const char*>(p) + bytes - 1};
-    for (const char* q : ends) {
-        cudaPointerAttributes at{};
-        if (cudaPointerGetAttributes(&at, q) != cudaSuccess) {
-            cudaGetLastError();
-            return false;
-        }
-        if (at.type != cudaMemoryTypeHost || at.devicePointer != q) return false;
+    cudaPointerAttributes at{};
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
     }
-    return true;
+    if (at.type != cudaMemoryTypeHost || at.devicePointer != p) return false;
+    using Get = CUresult(CUDAAPI*)(void*, CUpointer_attribute, CUdeviceptr);
+    static const Get get = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult r;
+        if (cudaGetDriverEntryPointByVersion("cuPointerGetAttribute", &f, 12000, cudaEnableDefault, &r) != cudaSuccess) {
+            cudaGetLastError();
+            f = nullptr;
+        }
+        return reinterpret_cast<Get>(f);
+    }();
+    const CUdeviceptr q = reinterpret_cast<CUdeviceptr>(p);
+    CUdeviceptr start = 0;
+    size_t size = 0;
+    return get && get(&start, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, q) == CUDA_SUCCESS &&
+           get(&size, CU_POINTER_ATTRIBUTE_RANGE_SIZE, q) == CUDA_SUCCESS && q >= start && q - start <= size &&
+           bytes <= size - (q - start);
 }
 
 int serve_fail(const std::string& m) { return ag_internal_fail(m.c_str()); }

@@ -265,7 +265,11 @@ typedef struct AetherServeRequest {
     const uint64_t* keys;
     uint32_t n_keys;
     uint32_t reserved;
-    void* host_out;       /* optional: the output planes are copied here (comps * out_pitch elements) */
+    void* host_out;       /* optional: receives the output planes, comps * out_pitch elements with out_pitch = n
+                             rounded up to a multiple of 32; complete when the request is done. What the samples
+                             n .. out_pitch - 1 of a plane hold is unspecified: outputs of up to 8 MiB in mapped
+                             pinned memory that are not kept are written by the kernel itself, which leaves
+                             them as they were; others are copied whole */
     uint64_t arrival_ns;  /* aether_serve_feed: arrival time after the feed starts */
 } AetherServeRequest;
 
