@@ -444,15 +444,16 @@ AG_EXPORT int aether_plan_source(void* plan, char* buf, size_t cap, size_t* len)
 // 256 and 64 threads: FP64 grade 25.1, 21.1 and 21.0 us, native 33.4, 24.5 and
 // 24.5), the others 16 (3x3 inverses, 4099 samples: 4.9 us at 256 and 3.5 at 64;
 // sums of 65536 terms 14.4 and 11.4 us), or 8 with four samples a thread (a b - c d
-// over 2^20 f32: 2.6 us at 256 and 128, 3.2 at 64).
+// over 2^20 f32: 2.6 us at 256 and 128, 3.2 at 64), and draws 3 (six lognormal ones
+// a sample in double-float, 2^20 samples: 85 us at 256, 97 at 128).
 PlanShape plan_shape(const PlanObj& P, uint64_t n, bool vectorized) {
     const uint64_t lanes = uint64_t(P.low.ipt) * uint64_t(vectorized ? P.vec : 1);
     int block = P.low.block, i = 0;
     if (P.low.by_size) {
         for (i = kNumBlocks - 1; i > 0; --i) {
-            if (kBlocks[i] > P.low.block || (kBlocks[i] == 512 && !P.tf)) continue;
+            if (kBlocks[i] > P.low.block || (kBlocks[i] == 512 && !P.tf && P.low.block > 512)) continue;
             const int bps = vectorized ? P.blocks_per_sm_v[i] : P.blocks_per_sm_s[i];
-            const uint64_t want = uint64_t(kBlocks[i] == 768 ? 24 * std::max(bps, 1) : P.tf ? 4 : lanes >= 4 ? 8 : 16) * uint64_t(P.sms);
+            const uint64_t want = uint64_t(kBlocks[i] == 768 || (kBlocks[i] == 512 && !P.tf) ? 24 * std::max(bps, 1) : P.tf ? 4 : P.plan.has_random ? 3 : lanes >= 4 ? 8 : 16) * uint64_t(P.sms);
             if ((n + kBlocks[i] * lanes - 1) / (kBlocks[i] * lanes) >= want) break;
         }
         block = kBlocks[i];

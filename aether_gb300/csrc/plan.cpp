@@ -1110,6 +1110,9 @@ int default_block(const Plan& P, int math) {
     // squeezed into 80 registers).
     const bool tf = triple_float(P, math);
     if (P.wants_sum() || (math == 0 && !tf) || (P.has_random && !heavy(P))) return 256;
+    // two draws a sample in double-float, 2^24 samples: N(0, 1) 281 us compiled
+    // for 512 threads, 298 for 768 and 295 for 256; three: 417, 406 and 433
+    if (P.has_random && !tf && P.dst_comps == 2) return 512;
     // 768 threads leave a thread 80 registers: too few for a matrix of
     // triple-floats (3x3 inverses, 2^24: 894 us at 512 threads, 1065 at 768) and
     // for native trees on middling sizes (plain fused expression, 2^20 x 3: 62
@@ -1119,11 +1122,15 @@ int default_block(const Plan& P, int math) {
 
 bool two_samples(const Plan& P, int math) {
     const bool f64 = P.dst_dtype == DType::F64;
+    // Several draws a sample in double-float are bound by Philox and the tables,
+    // which pairs do not share, and the pairs' registers leave fewer warps: two N(0,
+    // 1) over 2^22 samples 75 us by sample and 83 in pairs, six 255 and 305.
+    if (math == 1 && P.has_random && heavy(P) && P.dst_comps > 1) return false;
     return ((math == 1 && f64) || (math == 2 && !f64) || triple_float(P, math)) && pairable(P);
 }
 
 uint64_t one_sample_limit(const Plan& P, int math) {
-    if (P.wants_sum() || !two_samples(P, math)) return 0;
+    if (P.wants_sum() || !two_samples(P, math) || (P.has_random && !heavy(P))) return 0;   // light fills are Philox
     return heavy(P) && !triple_float(P, math) ? 2048 : 512;
 }
 
