@@ -471,12 +471,12 @@ __device__ __forceinline__ tf exp_table(int k) {
     return mk3(tv.x, tv.y, tv.z);
 }
 __device__ __forceinline__ tf2 exp_table(i2 k) { return pair(exp_table(k.a), exp_table(k.b)); }
+// e^x = 2^(k >> 6) exp_mantissa(x, k), the mantissa in [1, 2) but for rounding.
 template <class F>
-__device__ __forceinline__ tfT<F> exp_(tfT<F> x, typename lanes<F>::flag& ok) {
-    e64::within(x.x, -55.0f, 87.0f, ok);
+__device__ __forceinline__ tfT<F> exp_mantissa(tfT<F> x, typename lanes<F>::whole& k) {
     const F kx = fmul(x.x, bc<F>(AG_TF_INV_LN2_64));
     const F kf = e64::rint_f(kx);
-    const typename lanes<F>::whole k = e64::rint_i(kx);
+    k = e64::rint_i(kx);
     const tfT<F> ln2 = mk3(bc<F>(AG_TF_LN2_64_X), bc<F>(AG_TF_LN2_64_Y), bc<F>(AG_TF_LN2_64_Z));
     const tfT<F> r = renorm(sub(x, mul(ln2, kf)));
     const dfT<F> rr = mk(r.x, r.y);
@@ -492,7 +492,13 @@ __device__ __forceinline__ tfT<F> exp_(tfT<F> x, typename lanes<F>::flag& ok) {
     const tfT<F> p = mk3(h.hi, m.hi, fadd(fadd(m.lo, r.z), P.lo));
     const tfT<F> T = t64::exp_table(k);
     // T >= 1 leads T p (|p| < 2^-7)
-    const tfT<F> res = add_lead(T, mul(T, p));
+    return add_lead(T, mul(T, p));
+}
+template <class F>
+__device__ __forceinline__ tfT<F> exp_(tfT<F> x, typename lanes<F>::flag& ok) {
+    e64::within(x.x, -55.0f, 87.0f, ok);
+    typename lanes<F>::whole k;
+    const tfT<F> res = exp_mantissa(x, k);
     return scale(res, e64::p2f(e64::exp_power(k)));
 }
 #define AG_T64_NATIVE1(NAME)                                                                   \
@@ -538,8 +544,9 @@ namespace y64 = t64;   // the spelling of a plan's two-sample code
 // boundary than the evaluation's own error is handed to the FP64 pipe. log,
 // log1p, exp, sin and cos are within 0.52 ulp, under CUDA's 1 to 2; sin and cos
 // 0.76 beside multiples of pi/2 (0.63 seen in 9 10^6 arguments as near as the
-// fast path takes). Arguments outside the triple-float range, zeros, infinities and NaN take CUDA's
-// function out of line. Measured: a + b c + sin(a) exp(-c c) over 2^20
+// fast path takes). Arguments outside the triple-float range are scaled into it
+// out of line (wide_* below); subnormals, overflow, infinities, NaN and sines
+// beyond 2^22 take CUDA's function there. Measured: a + b c + sin(a) exp(-c c) over 2^20
 // three-component samples, 232 us with CUDA's functions, 65 us with these; a
 // fill of 3 uniform components and one N(0, 1) draw for 10^7 samples, 1555 and
 // 267 us.
@@ -547,23 +554,22 @@ namespace y64 = t64;   // the spelling of a plan's two-sample code
 namespace n64 {
 using t64::tf;
 
-#if defined(__CUDACC__) || defined(__CUDACC_RTC__)
-#define AG_N64_NOINLINE __noinline__
 // Zeros answer at once: sparse data has many.
 __device__ __forceinline__ bool is_zero(double x) {
     return (((unsigned)__double2hiint(x) & 0x7fffffffu) | (unsigned)__double2loint(x)) == 0u;
 }
-__device__ AG_N64_NOINLINE double slow_sqrt(double x) { return is_zero(x) ? x : __dsqrt_rn(x); }
-__device__ AG_N64_NOINLINE double slow_rsqrt(double x) { return __ddiv_rn(1.0, __dsqrt_rn(x)); }
-__device__ AG_N64_NOINLINE double slow_div(double a, double b) {
-    const unsigned eb = ((unsigned)__double2hiint(b) >> 20) & 0x7ffu;
-    if (is_zero(a) && eb - 1u < 2046u)   // b is finite and normal
-        return __hiloint2double((__double2hiint(a) ^ __double2hiint(b)) & (int)0x80000000, 0);
-    return __ddiv_rn(a, b);
-}
-__device__ AG_N64_NOINLINE double slow_exp(double x) { return is_zero(x) ? 1.0 : ::exp(x); }
-__device__ AG_N64_NOINLINE double slow_log(double x) { return ::log(x); }
-__device__ AG_N64_NOINLINE double slow_log1p(double x) { return is_zero(x) ? x : ::log1p(x); }
+#if defined(__CUDACC__) || defined(__CUDACC_RTC__)
+#define AG_N64_NOINLINE __noinline__
+__device__ __forceinline__ double slow_sqrt(double x) { return __dsqrt_rn(x); }
+__device__ __forceinline__ double slow_rsqrt(double x) { return __ddiv_rn(1.0, __dsqrt_rn(x)); }
+__device__ __forceinline__ double slow_div(double a, double b) { return __ddiv_rn(a, b); }
+__device__ __forceinline__ double slow_exp(double x) { return ::exp(x); }
+__device__ __forceinline__ double slow_log(double x) { return ::log(x); }
+__device__ __forceinline__ double slow_log1p(double x) { return ::log1p(x); }
+__device__ __forceinline__ double fma_rn(double x, double y, double z) { return __fma_rn(x, y, z); }
+#else
+#define AG_N64_NOINLINE inline
+inline double fma_rn(double x, double y, double z) { return std::fma(x, y, z); }
 #endif
 
 using e64::d2;
@@ -655,20 +661,101 @@ __device__ __forceinline__ auto log1p_core(tfT<F> a, typename lanes<F>::flag& ok
     e64::within(a.x, -0.75f, 3e38f, ok);   // nearer to -1 the reduced argument cancels
     return join(t64::log_s<false, t64::LOG_S1>(bc<F>(1.0f), a));
 }
+// Arguments the triple-float split does not take, out of line: the double is
+// brought to an exponent near 0 in integers, the same evaluation runs on it, and
+// the exponent goes back into the result's bits. What is left (values beside a
+// rounding boundary, subnormals, overflow, negative or non-finite arguments) is
+// CUDA's function's. sqrt of 3 x 2^22 doubles near 1e-20: 93 us, CUDA's
+// 187, near 1 50; quotients 132, 183 and 66; exp of -200 to -60 190 and 370; logarithms
+// near 1e25 184 and 705; sines up to 1e5 249 and 434 (ag_tf64_trig.cuh).
+__device__ __forceinline__ unsigned exponent(double x) { return ((unsigned)__double2hiint(x) >> 20) & 0x7ffu; }
+// exponent + k, mantissa and sign unchanged
+__device__ __forceinline__ double times_2(double x, int k) {
+    return __hiloint2double(__double2hiint(x) + (int)((unsigned)k << 20), __double2loint(x));
+}
+__device__ __forceinline__ bool normal_exponent(int e) { return (unsigned)(e - 1) < 2046u; }
+__device__ __forceinline__ bool in_split(unsigned e) { return e - 983u <= 100u; }   // |x| in [2^-40, 2^61)
+__device__ AG_N64_NOINLINE double wide_sqrt(double x) {
+    if (is_zero(x)) return x;
+    const unsigned e = (unsigned)__double2hiint(x) >> 20;   // the sign is its top bit
+    if (in_split(e) || !normal_exponent((int)e)) return slow_sqrt(x);
+    const int k = ((int)e - 1023) & ~1;
+    bool ok = true;
+    const tf a = split(times_2(x, -k), ok);
+    const double r = sqrt_core(a, ok);
+    return ok ? times_2(r, k / 2) : slow_sqrt(x);
+}
+__device__ AG_N64_NOINLINE double wide_rsqrt(double x) {
+    const unsigned e = (unsigned)__double2hiint(x) >> 20;
+    if (in_split(e) || !normal_exponent((int)e)) return slow_rsqrt(x);
+    const int k = ((int)e - 1023) & ~1;
+    bool ok = true;
+    const tf a = split(times_2(x, -k), ok);
+    const double r = rsqrt_core(a, ok);
+    return ok ? times_2(r, -(k / 2)) : slow_rsqrt(x);
+}
+__device__ AG_N64_NOINLINE double wide_div(double x, double y) {
+    const int ex = (int)exponent(x), ey = (int)exponent(y), k = ex - ey;
+    if (is_zero(x) && normal_exponent(ey)) return __hiloint2double((__double2hiint(x) ^ __double2hiint(y)) & (int)0x80000000, 0);
+    // both in the split's range and the quotient in div_core's: beside a boundary
+    const bool near = in_split((unsigned)ex) && in_split((unsigned)ey) && k > -64 && k < 95;
+    if (near || !normal_exponent(ex) || !normal_exponent(ey)) return slow_div(x, y);
+    bool ok = true;
+    const tf a = split(times_2(x, 1023 - ex), ok), b = split(times_2(y, 1023 - ey), ok);
+    const double r = div_core(a, b, ok);
+    return ok && normal_exponent((int)exponent(r) + k) ? times_2(r, k) : slow_div(x, y);
+}
+// Below 2^-40, e^x = 1 + x to 2^-81; elsewhere the power of two joins the bits.
+__device__ AG_N64_NOINLINE double wide_exp(double x) {
+    const unsigned e = exponent(x);
+    if (e < 983u) return __dadd_rn(1.0, x);
+    bool ok = e < 1033u;   // |x| < 2^10: the multiple of ln2/64 is exact
+    const tf a = split(x, ok);
+    int k;
+    const double r = join(t64::exp_mantissa(a, k));
+    return ok && normal_exponent((int)exponent(r) + (k >> 6)) ? times_2(r, k >> 6) : slow_exp(x);
+}
+// log x = k ln2 + log(x 2^-k); outside the split's range the first term leads.
+__device__ AG_N64_NOINLINE double wide_log(double x) {
+    const unsigned e = (unsigned)__double2hiint(x) >> 20;
+    if (in_split(e) || !normal_exponent((int)e)) return slow_log(x);
+    const int k = (int)e - 1023;
+    bool ok = true;
+    const tf a = split(times_2(x, -k), ok);
+    const tf ln2 = t64::mk3(64.0f * AG_TF_LN2_64_X, 64.0f * AG_TF_LN2_64_Y, 64.0f * AG_TF_LN2_64_Z);
+    return join(t64::add_lead(t64::mul(ln2, (float)k), t64::log_s<false, t64::LOG_S0>(0.0f, a)));
+}
+// Below 2^-40, log(1 + x) = x - x^2/2 to 2^-81 of it; above 2^60 it is log x to
+// 2^-13 of an ulp; between -1 and -1/2, 1 + x is exact.
+__device__ AG_N64_NOINLINE double wide_log1p(double x) {
+    const unsigned e = exponent(x);
+    if (is_zero(x)) return x;
+    if (e < 983u) return fma_rn(__dmul_rn(x, -0.5), x, x);
+    if (x > 0.0 && e < 2047u && !in_split(e)) return wide_log(x);
+    if (x > -1.0 && x <= -0.5) {
+        const double y = __dadd_rn(1.0, x);
+        if (!in_split(exponent(y))) return wide_log(y);
+        bool ok = true;
+        const tf a = split(y, ok);
+        const double r = log_core(a, ok);
+        if (ok) return r;
+    }
+    return slow_log1p(x);
+}
 #define AG_N64_FUNCTION(NAME)                                              \
     __device__ __forceinline__ double NAME(double x) {                     \
         bool ok = true;                                                    \
         const tf a = split(x, ok);                                         \
         const double r = NAME##_core(a, ok);                               \
-        return ok ? r : slow_##NAME(x);                                    \
+        return ok ? r : wide_##NAME(x);                                    \
     }                                                                      \
     __device__ __forceinline__ d2 NAME(d2 x) {                             \
         b2 ok{true, true};                                                 \
         const t64::tf2 a = split(x, ok);                                   \
         d2 r = NAME##_core(a, ok);                                         \
         if (!(ok.a && ok.b)) {                                             \
-            if (!ok.a) r.a = slow_##NAME(x.a);                             \
-            if (!ok.b) r.b = slow_##NAME(x.b);                             \
+            if (!ok.a) r.a = wide_##NAME(x.a);                             \
+            if (!ok.b) r.b = wide_##NAME(x.b);                             \
         }                                                                  \
         return r;                                                          \
     }
@@ -681,15 +768,15 @@ __device__ __forceinline__ double div(double x, double y) {
     bool ok = true;
     const tf a = split(x, ok), b = split(y, ok);
     const double r = div_core(a, b, ok);
-    return ok ? r : slow_div(x, y);
+    return ok ? r : wide_div(x, y);
 }
 __device__ __forceinline__ d2 div(d2 x, d2 y) {
     b2 ok{true, true};
     const t64::tf2 a = split(x, ok), b = split(y, ok);
     d2 r = div_core(a, b, ok);
     if (!(ok.a && ok.b)) {
-        if (!ok.a) r.a = slow_div(x.a, y.a);
-        if (!ok.b) r.b = slow_div(x.b, y.b);
+        if (!ok.a) r.a = wide_div(x.a, y.a);
+        if (!ok.b) r.b = wide_div(x.b, y.b);
     }
     return r;
 }

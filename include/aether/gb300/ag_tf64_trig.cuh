@@ -62,6 +62,28 @@ __device__ __forceinline__ tfT<F> reduce_pio2(tfT<F> x, typename lanes<F>::whole
     return renorm(r);
 }
 
+// r = x - q pi/2 for 2^10 <= |x| < 2^22, pi/2 as four floats, each the nearest
+// to what the ones before it leave (103 bits). x.x - q C0 is exact (Sterbenz)
+// but for q C0's rounding error, and its sum with x's other floats has at most
+// 53 bits, two floats; q C1 and q C2 join as exact pairs. The sums' third floats
+// round at 2^-73 in all, 2^-59 of |r| >= 2^-14; nearer arguments are flagged.
+__device__ __forceinline__ tf reduce_wide(tf x, int& q, bool& ok) {
+    const float qh = __fmul_rn(x.x, AG_TF_2OPI);
+    const float ql = __fmaf_rn(x.y, AG_TF_2OPI, __fmaf_rn(x.x, 2.5682553e-08f, __fmaf_rn(x.x, AG_TF_2OPI, -qh)));
+    const float q0 = e64::rint_f(qh);
+    const float qf = __fadd_rn(q0, e64::rint_f(__fadd_rn(__fsub_rn(qh, q0), ql)));
+    q = e64::rint_i(qf);
+    const df p0 = two_prod(qf, 1.57079637f), p1 = two_prod(qf, -4.37113883e-08f), p2 = two_prod(qf, -1.71512451e-15f);
+    const df s = two_sum(x.y, x.z), w = two_sum(__fsub_rn(x.x, p0.hi), s.hi);
+    tf r = mk3(w.hi, __fadd_rn(w.lo, s.lo), 0.0f);
+    r = add(r, mk3(-p0.lo, 0.0f, 0.0f));
+    r = add(r, mk3(-p1.hi, -p1.lo, 0.0f));
+    r = add(r, mk3(-p2.hi, -__fmaf_rn(qf, 1.0562999e-23f, p2.lo), 0.0f));
+    r = renorm(r);
+    ok = ok && fabsf(r.x) >= 6.103515625e-5f;
+    return r;
+}
+
 // The table row of j/2048 at quadrant q: the pair (A, B) and the sign of the
 // wanted output. By quadrant it is +-sin r or +-cos r, and both are
 // A (1 + cm1) + B st with (A, B) = (S, C) for sin r and (C, -S) for cos r, so
@@ -89,9 +111,7 @@ __device__ __forceinline__ tf2 neg_if(b2 c, tf2 v) { return pair(neg_if(c.a, ln0
 
 // One output of sin/cos at x = q pi/2 + r.
 template <class F>
-__device__ __forceinline__ tfT<F> trig_(tfT<F> x, bool want_cos, typename lanes<F>::flag& ok) {
-    typename lanes<F>::whole q;
-    const tfT<F> r = reduce_pio2(x, q, ok);
+__device__ __forceinline__ tfT<F> trig_reduced(tfT<F> r, typename lanes<F>::whole q, bool want_cos) {
     const F jx = fmul(r.x, bc<F>(2048.0f));
     const F jf = e64::rint_f(jx);
     // t = r - j/2048: the leading difference is exact (Sterbenz, or j = 0)
@@ -116,6 +136,12 @@ __device__ __forceinline__ tfT<F> trig_(tfT<F> x, bool want_cos, typename lanes<
     return neg_if(R.minus, v);
 }
 template <class F>
+__device__ __forceinline__ tfT<F> trig_(tfT<F> x, bool want_cos, typename lanes<F>::flag& ok) {
+    typename lanes<F>::whole q;
+    const tfT<F> r = reduce_pio2(x, q, ok);
+    return trig_reduced(r, q, want_cos);
+}
+template <class F>
 __device__ __forceinline__ tfT<F> sin_(tfT<F> x, typename lanes<F>::flag& ok) {
     return trig_(x, false, ok);
 }
@@ -129,8 +155,8 @@ __device__ __forceinline__ tfT<F> cos_(tfT<F> x, typename lanes<F>::flag& ok) {
 #if defined(__CUDACC__) || defined(__CUDACC_RTC__) || defined(AG_N64_HOST_CHECK)
 namespace n64 {
 #if defined(__CUDACC__) || defined(__CUDACC_RTC__)
-__device__ AG_N64_NOINLINE double slow_sin(double x) { return ::sin(x); }
-__device__ AG_N64_NOINLINE double slow_cos(double x) { return ::cos(x); }
+__device__ __forceinline__ double slow_sin(double x) { return ::sin(x); }
+__device__ __forceinline__ double slow_cos(double x) { return ::cos(x); }
 __device__ AG_N64_NOINLINE double slow_normal(ag_u64 seed, ag_u32 g, ag_u32 c) { return ag::normal_f64(seed, g, c); }
 #endif
 template <class F>
@@ -141,6 +167,18 @@ template <class F>
 __device__ __forceinline__ auto cos_core(tfT<F> a, typename lanes<F>::flag& ok) {
     return join(t64::cos_(a, ok));
 }
+// Arguments that sin_core and cos_core flag, out of line.
+#define AG_N64_WIDE_TRIG(NAME, COS)                                        \
+    __device__ AG_N64_NOINLINE double wide_##NAME(double x) {              \
+        bool ok = exponent(x) - 1033u < 12u;   /* |x| in [2^10, 2^22) */   \
+        if (!ok) return slow_##NAME(x);                                    \
+        int q;                                                             \
+        const tf r = t64::reduce_wide(split(x, ok), q, ok);                \
+        const double v = join(t64::trig_reduced(r, q, COS));               \
+        return ok ? v : slow_##NAME(x);                                    \
+    }
+AG_N64_WIDE_TRIG(sin, false)
+AG_N64_WIDE_TRIG(cos, true)
 // Below 2^-27, sin x = x and cos x = 1 to a quarter of an ulp.
 __device__ __forceinline__ bool tiny(double x) {
     return ((unsigned)__double2hiint(x) & 0x7fffffffu) < (996u << 20);
@@ -150,10 +188,10 @@ __device__ __forceinline__ bool tiny(double x) {
         bool ok = true;                                                    \
         const tf a = split(x, ok);                                         \
         const double r = NAME##_core(a, ok);                               \
-        return tiny(x) ? (SMALL) : ok ? r : slow_##NAME(x);                \
+        return tiny(x) ? (SMALL) : ok ? r : wide_##NAME(x);                \
     }                                                                      \
     __device__ __forceinline__ double NAME##_rest(double x) {              \
-        return tiny(x) ? (SMALL) : slow_##NAME(x);                         \
+        return tiny(x) ? (SMALL) : wide_##NAME(x);                         \
     }                                                                      \
     __device__ __forceinline__ d2 NAME(d2 x) {                             \
         b2 ok{true, true};                                                 \
