@@ -354,7 +354,8 @@ def assign_sub(dst, expr, **kw):
 
 def global_sum(expr, n, dtype="f64", stream=None, workspace=None, **kw):
     """Compensated sum over samples of a rank-0 expression: returns a device
-    tensor (hi, comp), reduced in a fixed order (deterministic)."""
+    tensor (hi, comp), reduced in an order that the device and the plan's
+    lowering fix (the same bits on every run)."""
     torch = _torch()
     out = torch.zeros(2, dtype=torch.float64, device="cuda")
     L = prepare((dtype, ()), expr, op="sum", n=n, reduce_out=out, workspace=workspace, **kw)

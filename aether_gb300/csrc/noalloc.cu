@@ -1,7 +1,7 @@
 // noalloc.cu -- launching a sum plan without any device allocation.
 //
 // A sum plan needs device scratch: a completion counter plus one (hi, comp)
-// partial per chunk of samples. aether_plan_launch takes it from the caller
+// partial per CTA, at most one per chunk of samples. aether_plan_launch takes it from the caller
 // or allocates it for the plan on first use. Some callers cannot allocate at
 // the point where they launch: hosts that run under a fixed device-memory
 // budget (a serving loop that admits work by bytes) must not grow it behind

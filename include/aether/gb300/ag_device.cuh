@@ -32,7 +32,7 @@ struct AgArgs {
     float scl[AG_MAX_SC];         // for plans lowered to emulated FP64
     ag_u64 key[AG_MAX_KEYS];      // generator keys of random leaves
     double* red;                  // sum plans: (hi, comp) result
-    char* ws;                     // sum plans: counter + per-chunk partials
+    char* ws;                     // sum plans: counter + one partial per CTA
     ag_u64 ws_bytes;
 };
 static_assert(sizeof(AgArgs) == 632, "AgArgs layout must match the host image in abi.cpp");

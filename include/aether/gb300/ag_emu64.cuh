@@ -1,13 +1,15 @@
 // ag_emu64.cuh -- FP64 expression math on the FP32 and integer pipes.
 //
-// Included by generated kernels lowered with math = 1. On GB300 the FP64 pipe
+// Included by generated kernels lowered with math = 1, 2 or 3, and by native ones
+// through ag_tf64.cuh. On GB300 the FP64 pipe
 // issues about 1.6 operations per clock per SM against about 110 FFMA and 59
 // IMAD (double <-> float conversions run on the FP64 pipe as well), so an
 // FP64 expression kernel with transcendental nodes is bound by that pipe long
 // before HBM. Here every double is split into a double-float pair
 // (hi + lo, two floats, about 48 significant bits) with integer operations,
 // the expression is evaluated in double-float arithmetic, and each output is
-// reassembled into a double with one FP64 addition.
+// reassembled into a double: with one FP64 addition (to_double) where a
+// transcendental node hides it, in integers (out_double, out_join) elsewhere.
 //
 // Accuracy: relative error about 2^-46 per function (a few tens of double
 // ulps in the worst case), against 2^-53 for the native pipe. Samples whose

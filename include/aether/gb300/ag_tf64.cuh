@@ -1,13 +1,15 @@
 // ag_tf64.cuh -- FP64-grade expression math on the FP32 and integer pipes.
 //
-// Included by generated kernels lowered with math = 3. The double-float
+// Included by generated kernels lowered with math = 3, and by native ones (math =
+// 0, and the native lanes of the others) that divide, take a root, exp, log, sine
+// or cosine, or draw a normal (ag::n64 below). The double-float
 // lowering (ag_emu64.cuh, math = 1) carries about 48 significant bits, tens
 // of double ulps short of the FP64 contract; the native pipe meets the
 // contract at a few per cent of HBM bandwidth. Here every double is split
 // exactly into three floats (24 + 23 + 6 significant bits, integer operations
 // only), the expression is evaluated in triple-float arithmetic (about 72
 // bits, of which the operations keep well over 60), and each output is
-// reassembled into a double with two FP64 additions, one rounding of a value
+// reassembled into a double in integers (out_double), one rounding of a value
 // already exact to far below half an ulp.
 //
 // Representation: v = x + y + z with |y| of the order of ulp(x) and |z| of
@@ -16,7 +18,9 @@
 // accumulated with plain float operations, whose roundings (2^-24 of a term
 // of 2^-47 of the value) stay near 2^-71. The components are not kept
 // strictly non-overlapping: every operation below accepts a y up to a few
-// ulps of x and a z up to a few ulps of y.
+// ulps of x and a z up to a few ulps of y. A sum that cancels leaves z large
+// beside x, with the absolute error of its operands' scale; the generator
+// renormalises such a value before it is reassembled.
 //
 // Range: inputs with magnitudes in [2^-40, 2^60] (and products the generator
 // cannot prove to stay above 2^-80) keep every component a normal float;

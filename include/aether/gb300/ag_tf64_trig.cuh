@@ -1,7 +1,7 @@
 // ag_tf64_trig.cuh -- FP64-grade sine and cosine in triple-float arithmetic.
 //
-// Included by generated FP64-grade kernels (math = 3) with trigonometric
-// nodes. x = q pi/2 + r with pi/2 in four parts (the first with 14 significant
+// Included by generated FP64-grade and native kernels with trigonometric nodes or
+// normal draws. x = q pi/2 + r with pi/2 in four parts (the first with 14 significant
 // bits, so q P0 is exact for |q| < 2^10; about 87 bits in all); r = j/2048 + t
 // with |t| <= 2^-12 and S_j, C_j = sin, cos(j/2048) from a table of three
 // floats each; then, by quadrant, sin r = S (1 + cm1) + C st and

@@ -99,7 +99,8 @@ typedef struct AetherLaunch {
     uint32_t n_scalars;
     const uint64_t* keys;         /* Generator keys of random leaves (random/Generator.h:183) */
     uint32_t n_keys;
-    double* reduce_out;           /* sum plans: device pointer to (hi, comp) */
+    double* reduce_out;           /* sum plans: device pointer to (hi, comp): the same bits on every run of a
+                                     plan on one kind of device and build, whose grid groups the terms */
     /* Sum plans: device scratch of aether_plan_workspace_size bytes, or NULL
      * for one of the plan's own. Own workspaces form a pool: a launch reuses
      * an entry last used on the same stream or one whose last launch has
@@ -114,7 +115,7 @@ typedef struct AetherLaunch {
 
 /* Lowering options; any field <= 0 takes the tuned default. */
 typedef struct AetherLowering {
-    int block;        /* threads per CTA */
+    int block;        /* threads per CTA; unnamed (as ipt, vec and min_blocks are), each launch chooses by its size */
     int ipt;          /* lane groups per thread per chunk */
     int vec;          /* samples per lane group (vector width) */
     int contract;     /* 1: FMA contraction allowed, 0: every add/mul rounds (-fmad=false), -1: default (1) */
@@ -134,7 +135,7 @@ typedef struct AetherPlanInfo {
     int dst_comps;
     int dst_dtype;            /* 0 f64, 1 f32, 2 ff */
     int is_sum;               /* writes a (hi, comp) global sum */
-    int block, ipt, vec;
+    int block, ipt, vec;      /* block: the most threads a launch's CTAs have */
     int registers;            /* per thread, of the vectorized kernel */
     int blocks_per_sm;        /* occupancy of the vectorized kernel */
     double compile_ms;        /* 0 when the kernel came from a cache */
@@ -175,7 +176,7 @@ typedef struct AetherBatchInfo {
     double compile_ms;
 } AetherBatchInfo;
 
-/* Compile one persistent kernel for `plans` (block/ipt from `lowering`). */
+/* Compile one persistent kernel for `plans` (block/ipt from `lowering`; unset: 128, 1). */
 int aether_batch_create(void* const* plans, int n_plans, const AetherLowering* lowering, void** batch);
 /* Replace the work list; items are cut into equal tiles the CTAs take
  * round-robin. Returns once the list is on the device. */
@@ -239,7 +240,8 @@ typedef struct AetherServeConfig {
     int mode;                  /* AETHER_SERVE_BATCHED or AETHER_SERVE_PLAIN */
     int max_inflight;          /* launches on the device at once; 0 = 4 */
     int max_items;             /* requests per batched launch; 0 = 256 */
-    int block, ipt;            /* lowering of the batched kernel; 0 = 512, 1 */
+    int block, ipt;            /* lowering of the work-list kernels; 0 = the plan's own where it names one, else
+                                  128 and 1 (grouping 1: 512 and 1) */
     int idle_spin_us;          /* the loop polls this long after its last work before it sleeps; 0 = 2000 */
     int upload_engine;         /* 0: SMs read mapped pinned host operands in one gather kernel per launch
                                   (other memory: copy engine); 1: copy engine only */
