@@ -1117,7 +1117,10 @@ int default_block(const Plan& P, int math) {
     // triple-floats (3x3 inverses, 2^24: 894 us at 512 threads, 1065 at 768) and
     // for native trees on middling sizes (plain fused expression, 2^20 x 3: 62
     // us with 112 registers, 66 with 80)
-    return tf && (math == 0 || P.dst_comps >= 9) ? 512 : 768;
+    if (tf && (math == 0 || P.dst_comps >= 9)) return 512;
+    // six and more components with a function always spill at 768 (narrower_block
+    // would compile them again)
+    return heavy(P) && !P.has_random && P.dst_comps >= 6 ? 512 : 768;
 }
 
 bool two_samples(const Plan& P, int math) {
