@@ -523,34 +523,42 @@ struct Gen {
         }
         return sum_only_memo[size_t(id)] != 0;
     }
-    // Triple-floats: whether node `id`'s lower floats may overlap its upper ones
-    // by more than a few bits. A sum that cancels leaves them so, and products,
-    // quotients and roots of such a value do too; functions that reduce their
-    // argument do not.
+    // Triple-floats: how far node `id`'s lower floats may overlap its upper ones.
+    // 0: by a few bits. 3: the third float reaches into the second (exp adds the low
+    // part of a double-float series, 2^-39 of the value, as the third). 2: so does
+    // log's, by 2^-35 of the reduced logarithm, mostly a small part of the whole; 1:
+    // a sum of one sign with only one such operand, where it is rarer still. 4: by
+    // any amount (a sum that cancelled). Products, quotients, roots and other sums of
+    // one sign pass on what their operands have.
     std::vector<signed char> overlap_memo;
-    bool overlaps(int id) {
-        static const std::set<std::string> none = {"in", "sc", "lit", "lognormal", "exponential", "bernoulli",
-                                                   "pow", "pows", "atan2", "hypot"};
+    int overlap(int id) {
+        static const std::set<std::string> none = {"in", "sc", "lit", "bernoulli", "pow", "pows", "atan2", "hypot"};
+        static const std::set<std::string> logs = {"log", "log1p", "exponential"};
         static const std::set<std::string> as_kids = {
             "bcast", "at0", "comp", "seg", "row", "col", "transpose", "block", "reshape", "stack", "neg", "abs", "qconj",
             "pureq", "select", "min", "max", "mins", "maxs", "clamp", "sq", "mul", "scale", "outer", "div", "sqrt",
             "rsqrt", "sqnorm", "norm", "rnorm", "unit", "maxnorm"};
         if (overlap_memo.empty()) overlap_memo.assign(P.nodes.size(), -1);
         signed char& m = overlap_memo[size_t(id)];
-        if (m >= 0) return m != 0;
+        if (m >= 0) return m;
         const Node& n = P.nodes[size_t(id)];
         const std::string& op = n.op;
-        bool r = true;
+        int r = 4;
         if (as_kids.count(op) || (op == "add" && nonneg(n.kids[0]) && nonneg(n.kids[1]))) {
-            r = false;
-            for (size_t j = op == "select" ? 1 : 0; j < n.kids.size(); ++j) r = r || overlaps(n.kids[j]);
+            r = 0;
+            for (size_t j = op == "select" ? 1 : 0; j < n.kids.size(); ++j) r = std::max(r, overlap(n.kids[j]));
+            if (op == "add" && r == 2 && std::min(overlap(n.kids[0]), overlap(n.kids[1])) < 2) r = 1;
+        } else if (op == "exp" || op == "lognormal") {
+            r = 3;
+        } else if (logs.count(op)) {
+            r = 2;
         } else if (op == "normal") {   // N(0, 1) is the draw itself
             const Node &mean = P.nodes[size_t(n.kids[0])], &dev = P.nodes[size_t(n.kids[1])];
-            r = !(mean.op == "lit" && mean.lit == 0.0 && dev.op == "lit" && dev.lit == 1.0);
+            r = mean.op == "lit" && mean.lit == 0.0 && dev.op == "lit" && dev.lit == 1.0 ? 0 : 4;
         } else if (none.count(op) || unary_ops().count(op)) {
-            r = false;
+            r = 0;
         }
-        m = r ? 1 : 0;
+        m = (signed char)r;
         return r;
     }
     std::string sqr(bool u, const std::string& x) { return (u ? NS + "sqr_u(" : NS + "sqr(") + x + ")"; }
@@ -1287,15 +1295,17 @@ std::string generate_source(const Plan& plan_in, const Lowering& low, const std:
     const bool joins = tfx || (!prec && !heavy(P));
     // The output range test is left out when the magnitude bounds of the root
     // keep every value of a lane that passed its other checks inside [2^-88,
-    // 2^126) (2^-80 for triple-floats). Either reassembly is right for every
-    // value, a NaN (the root of a negative number) among them.
+    // 2^126) (2^-80 for triple-floats), zeros and NaN (the root of a negative
+    // number) aside.
     auto out_safe = [&](Gen& G) { return emu && G.lo_of(P.root) >= (tfx ? -80 : -88) && G.hi_of(P.root) <= 125; };
-    // The reassembly of v, and the range test before it (out_double of a
-    // triple-float holds its own).
+    // The reassembly of v, and the range test before it (a triple-float's holds
+    // its own, and so does that of a bounded root).
     auto dbl_out = [&](Gen& G, const std::string& v) -> std::string {
-        if (tfx)
-            return G.NS + "out_double(" + (G.overlaps(P.root) ? G.NS + "renorm(" + v + ")" : v) + (out_safe(G) ? ")" : ", ok_)");
-        return G.NS + (!joins ? "to_double(" : out_safe(G) ? "out_double(" : "out_join(") + v + ")";
+        if (!joins) return G.NS + "to_double(" + v + ")";
+        const int k = tfx ? G.overlap(P.root) : 0;
+        const std::string w = k == 4 ? G.NS + "renorm(" + v + ")" : k >= 2 ? G.NS + "tail(" + v + ")" : v;
+        const std::string fn = (out_safe(G) ? "out_bounded" : "out_double") + std::string(k == 1 ? "<true>(" : "(");
+        return G.NS + fn + w + (tfx || out_safe(G) ? ", ok_)" : ")");
     };
     auto dbl_test = [&](Gen& G, const std::string& v) -> std::string {
         if (tfx || out_safe(G)) return "";

@@ -9,7 +9,7 @@
 // (hi + lo, two floats, about 48 significant bits) with integer operations,
 // the expression is evaluated in double-float arithmetic, and each output is
 // reassembled into a double: with one FP64 addition (to_double) where a
-// transcendental node hides it, in integers (out_double, out_join) elsewhere.
+// transcendental node hides it, in integers (out_double) elsewhere.
 //
 // Accuracy: relative error about 2^-46 per function (a few tens of double
 // ulps in the worst case), against 2^-53 for the native pipe. Samples whose
@@ -413,6 +413,8 @@ __device__ __forceinline__ bool out_ok(df v) {
     const unsigned e = ((unsigned)__float_as_int(v.hi) >> 23) & 0xffu;
     return e - 37u <= 216u;   // |hi| in [2^-90, 2^127)
 }
+__device__ __forceinline__ bool all_of(bool x) { return x; }
+__device__ __forceinline__ bool all_of(b2 x) { return x.a && x.b; }
 __device__ __forceinline__ bool both_of(bool x, bool y) { return x && y; }
 __device__ __forceinline__ b2 both_of(b2 x, b2 y) { return b2{x.a && y.a, x.b && y.b}; }
 __device__ __forceinline__ b2 out_ok(df2 v) { return b2{out_ok(ln0(v)), out_ok(ln1(v))}; }
@@ -498,40 +500,32 @@ __device__ __forceinline__ b2 join_head(f2 x) {
 __device__ __forceinline__ int units_20(float x) { return to_int(__fmul_rn(x, 1048576.0f)); }
 __device__ __forceinline__ i2 units_20(f2 x) { return i2{units_20(ln0(x)), units_20(ln1(x))}; }
 template <class F>
-__device__ __forceinline__ auto out_join(dfT<F> v) {
+__device__ __forceinline__ auto out_double(dfT<F> v) {
     const dfT<F> n = fast_two_sum(v.hi, v.lo);   // |lo| <= half an ulp of hi: no carry past its binade
     return join_bits(n.hi, units_20(fmul(n.lo, join_scale<20>(n.hi, n.lo))));
 }
-#if defined(__CUDACC__) || defined(__CUDACC_RTC__)
-// Out of line: predicated, its FP64 operations would issue for every warp with
-// a zero in it.
-__device__ __noinline__ double slow_sum(float hi, float lo) { return to_double(mk(hi, lo)); }
-#else
-__device__ __forceinline__ double slow_sum(float hi, float lo) { return to_double(mk(hi, lo)); }
-#endif
-// Zeros, which sparse results have many of, need no sum.
-__device__ __forceinline__ void or_sum(bool fits, df v, double& r) {
-    if (!fits) {
-        const unsigned hb = (unsigned)__float_as_int(v.hi), lb = (unsigned)__float_as_int(v.lo);
-        r = __hiloint2double((int)(hb & lb), 0);
-        if (((hb | lb) & 0x7fffffffu) != 0u) r = slow_sum(v.hi, v.lo);
-    }
+// r, or the double of x where x is zero or NaN; `ok` is cleared where neither
+// that nor `fits` holds.
+__device__ __forceinline__ double or_zero_nan(float x, double r, bool fits, bool& ok) {
+    const unsigned xb = (unsigned)__float_as_int(x);
+    const bool keep = !(x > 0.0f || x < 0.0f);
+    ok = ok && (fits || keep);
+    return keep ? __hiloint2double((int)((xb & 0x80000000u) | ((xb & 0x7fffffffu) != 0u ? 0x7ff80000u : 0u)), 0) : r;
 }
-__device__ __forceinline__ void or_sum(b2 fits, df2 v, d2& r) {
-    if (!(fits.a && fits.b)) {
-        or_sum(fits.a, ln0(v), r.a);
-        or_sum(fits.b, ln1(v), r.b);
-    }
+__device__ __forceinline__ d2 or_zero_nan(f2 x, d2 r, b2 fits, b2& ok) {
+    return d2{or_zero_nan(ln0(x), r.a, fits.a, ok.a), or_zero_nan(ln1(x), r.b, fits.b, ok.b)};
 }
-// A plan's output, right for every value: heads out of range, zeros and NaN
-// take the FP64 sum.
+// A plan's output whose bounds keep it in range: zero and NaN (the root of a
+// negative number) leave as they are.
 template <class F>
-__device__ __forceinline__ auto out_double(dfT<F> v) {
-    auto r = out_join(v);
-    or_sum(join_head<20>(fadd(v.hi, v.lo)), v, r);
+__device__ __forceinline__ auto out_bounded(dfT<F> v, typename lanes<F>::flag& ok) {
+    const F n = fadd(v.hi, v.lo);
+    const typename lanes<F>::flag fits = join_head<20>(n);
+    auto r = out_double(v);
+    if (!all_of(fits)) r = or_zero_nan(n, r, fits, ok);
     return r;
 }
-// For values that may have left the range, out_join after this test: the lane
+// For values that may have left the range, out_double after this test: the lane
 // runs natively where it fails.
 template <class F>
 __device__ __forceinline__ void out_double_ok(dfT<F> v, typename lanes<F>::flag& ok) {

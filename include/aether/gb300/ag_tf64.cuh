@@ -211,6 +211,12 @@ __device__ __forceinline__ tfT<F> renorm(tfT<F> v) {
     const dfT<F> w = two_sum(v.x, s.hi);
     return mk3(w.hi, w.lo, s.lo);
 }
+// The same for y and z alone, of a value whose x leads its y already.
+template <class F>
+__device__ __forceinline__ tfT<F> tail(tfT<F> v) {
+    const dfT<F> s = two_sum(v.y, v.z);
+    return mk3(v.x, s.hi, s.lo);
+}
 
 // Reciprocal: the double-float reciprocal (about 2^-47) refined by one Newton
 // step r' = r + r e, e = 1 - y r. y r is within 2^-46 of 1, so 1 - x of the
@@ -798,46 +804,14 @@ __device__ __forceinline__ bool join_fits(float x, float Y, float Z) {
 __device__ __forceinline__ b2 join_fits(f2 x, f2 Y, f2 Z) {
     return b2{join_fits(ln0(x), ln0(Y), ln0(Z)), join_fits(ln1(x), ln1(Y), ln1(Z))};
 }
-#if defined(__CUDACC__) || defined(__CUDACC_RTC__)
-// Out of line: predicated, its five FP64 operations would issue for every warp
-// with a zero in it.
-__device__ __noinline__ double slow_sum(float x, float y, float z) { return to_double(mk3(x, y, z)); }
-#else
-__device__ __forceinline__ double slow_sum(float x, float y, float z) { return to_double(mk3(x, y, z)); }
-#endif
-// Zeros, which sparse results have many of, need no sum.
-__device__ __forceinline__ void or_sum(bool fits, tf v, double& r) {
-    if (!fits) {
-        const unsigned xb = (unsigned)__float_as_int(v.x), yb = (unsigned)__float_as_int(v.y), zb = (unsigned)__float_as_int(v.z);
-        r = __hiloint2double((int)(xb & yb & zb), 0);
-        if (((xb | yb | zb) & 0x7fffffffu) != 0u) r = slow_sum(v.x, v.y, v.z);
-    }
-}
-__device__ __forceinline__ void or_sum(bool fits, tf v, double& r, bool& ok) {
-    if (!fits) {
-        ok = ok && out_ok(v);
-        if (ok) r = slow_sum(v.x, v.y, v.z);
-    }
-}
-__device__ __forceinline__ void or_sum(b2 fits, tf2 v, e64::d2& r) {
-    if (!(fits.a && fits.b)) {
-        or_sum(fits.a, ln0(v), r.a);
-        or_sum(fits.b, ln1(v), r.b);
-    }
-}
-__device__ __forceinline__ void or_sum(b2 fits, tf2 v, e64::d2& r, b2& ok) {
-    if (!(fits.a && fits.b)) {
-        or_sum(fits.a, ln0(v), r.a, ok.a);
-        or_sum(fits.b, ln1(v), r.b, ok.b);
-    }
-}
-// A plan's output: x + y + z rounded once to nearest even, without the FP64
-// pipe (five operations of it in to_double) where the parts overlap no more
-// than an operation on normalised operands leaves them; to_double otherwise.
-// Right for every value; a sum that may cancel is handed over renormalised so
-// that it takes the integers (renorm is 12 FP32 operations). Y is rounded to an
-// even number of units and what is left by an addition to 1.5 2^22, whose last
-// place is half of Y's unit, so that a tie goes to the even double.
+// x + y + z rounded once to nearest even, without the FP64 pipe (five operations
+// of it in to_double), where join_fits holds: where the parts overlap no more
+// than a product or a root of normalised operands leaves them. The generator hands
+// over a sum that may cancel renormalised (12 FP32 operations), and what comes from
+// an exponential or a logarithm, whose third float is the rest of a double-float
+// series, with its tail renormalised (6). Y is rounded to an even number of
+// units and what is left by an addition to 1.5 2^22, whose last place is half of
+// Y's unit, so that a tie goes to the even double.
 __device__ __forceinline__ int half_units(float g) { return __float_as_int(__fadd_rn(g, 6291456.0f)) - 0x4AC00000; }
 __device__ __forceinline__ i2 half_units(f2 g) {
     const f2 t = fadd(g, bc<f2>(6291456.0f));
@@ -852,20 +826,40 @@ __device__ __forceinline__ auto out_join(tfT<F> v, typename lanes<F>::flag& fits
     fits = join_fits(v.x, Y, Z);
     return e64::join_bits(v.x, e64::plus(e64::plus(h, h), half_units(g)));
 }
-template <class F>
-__device__ __forceinline__ auto out_double(tfT<F> v) {
-    typename lanes<F>::flag fits;
-    auto r = out_join(v, fits);
-    or_sum(fits, v, r);
-    return r;
+// Where parts that seldom overlap did: the value with its tail renormalised.
+__device__ __forceinline__ void take(bool& fits, double& r, bool f, double v) {
+    if (!fits) r = v, fits = f;
 }
-// The same for a value that may have left the range: `ok` is cleared where
-// out_ok is false.
-template <class F>
+__device__ __forceinline__ void take(b2& fits, e64::d2& r, b2 f, e64::d2 v) {
+    take(fits.a, r.a, f.a, v.a);
+    take(fits.b, r.b, f.b, v.b);
+}
+template <class F, class D>
+__device__ AG_N64_NOINLINE void out_again(tfT<F> v, typename lanes<F>::flag& fits, D& r) {
+    typename lanes<F>::flag f;
+    const D w = out_join(tail(v), f);
+    take(fits, r, f, w);
+}
+// A plan's output. `ok` is cleared where the parts do not fit; the lane runs
+// natively there.
+template <bool RETRY = false, class F>
 __device__ __forceinline__ auto out_double(tfT<F> v, typename lanes<F>::flag& ok) {
     typename lanes<F>::flag fits;
     auto r = out_join(v, fits);
-    or_sum(fits, v, r, ok);
+    if (RETRY && !e64::all_of(fits)) out_again(v, fits, r);
+    ok = e64::both_of(ok, fits);
+    return r;
+}
+// The same for a root whose bounds keep it in range: zero and NaN (the root of a
+// negative number) leave as they are.
+template <bool RETRY = false, class F>
+__device__ __forceinline__ auto out_bounded(tfT<F> v, typename lanes<F>::flag& ok) {
+    typename lanes<F>::flag fits;
+    auto r = out_join(v, fits);
+    if (!e64::all_of(fits)) {
+        if (RETRY) out_again(v, fits, r);
+        r = e64::or_zero_nan(v.x, r, fits, ok);
+    }
     return r;
 }
 }  // namespace t64

@@ -50,8 +50,17 @@ struct Stat {
             return;
         }
         const double want = t64::to_double(v);
-        const e64::d2 p = t64::out_double(t64::pair(v, w)), q = t64::out_double(t64::pair(w, v));
-        const double got[3] = {t64::out_double(v), p.a, q.b};
+        bool ok = true;
+        e64::b2 po = {true, true}, qo = {true, true};
+        const double one = t64::out_double(v, ok);
+        const e64::d2 p = t64::out_double(t64::pair(v, w), po), q = t64::out_double(t64::pair(w, v), qo);
+        if (!ok) {
+            ++native;
+            differ += po.a || qo.b;
+            return;
+        }
+        differ += !(po.a && qo.b);
+        const double got[3] = {one, p.a, q.b};
         const Q exact = (Q)v.x + (Q)v.y + (Q)v.z;
         bool d = false;
         for (double g : got) {
@@ -86,7 +95,6 @@ int main() {
     // v as the generated code hands it over: sums go through renorm first
     auto sum = [&](Stat& s, tf v) {
         const tf r = t64::renorm(v);
-        s.add(v, last);
         s.add(r, last);
         last = r;
     };
@@ -124,6 +132,22 @@ int main() {
         const float h = (float)(sgn() * std::exp2(e)) * (i % 3 ? 1.0f : (float)(1.0 + 0.99 * u01(rng)));
         edge.add(t64::mk3(h, (float)(h * sgn() * logu(-40, -24.01)), 0.0f), last);
     }
+    // single operations as the generator hands them over: with their tail
+    // renormalised after an exponential or a logarithm, as they are elsewhere
+    Stat op[12], near;
+    for (long i = 0; i < 5 * N; ++i) {
+        const tf a = split(logu(-20, 20)), b = split(sgn() * logu(-20, 20)), c = split(logu(-2, 2)), d = split(logu(-2, 2));
+        bool ok = true;
+        const tf e = t64::exp_(split(sgn() * logu(-30, 5.5)), ok), l = t64::log_(split(logu(-30, 30))),
+                 p = t64::log1p_(split(logu(-30, 30)));
+        const tf v[12] = {t64::mul(a, b), t64::div(b, a), t64::recip(a), t64::sqrt_(a), t64::rsqrt_(a),
+                          t64::sqrt_(t64::add_fast(t64::sqr(c), t64::sqr(d))), t64::add_fast(c, d), a,
+                          t64::tail(e), t64::tail(l), t64::tail(p), t64::tail(t64::mul(e, l))};
+        for (int k = 0; k < 12; ++k) op[k].add(v[k], last);
+        near.add(t64::tail(t64::log_(split(1.0 + sgn() * logu(-50, -3)))), last);
+    }
+    line("near", 0, near);
+    for (int k = 0; k < 12; ++k) line("op", k, op[k]);
     line("ties", 0, ties);
     line("whole", 0, whole);
     line("heads", 0, heads);
